@@ -26,6 +26,7 @@
 #include "gemm.cuh"
 #include "sm100.cuh"
 #include "prof.cuh"
+#include "skinny.cuh"
 #include <atomic>
 #include <mutex>
 #include <string.h>
@@ -1026,6 +1027,17 @@ int mt_gemm_ex(const void* A, const void* B, void* C, void* preact, const void* 
   g.aux = aux;
   g.aux_mode = aux_mode;
   cudaStream_t st = as_stream(stream);
+  if (!g_force_simt && g_tile_policy == 0 && M <= kSkinnyMaxRows && !trans_a && trans_b && !accumulate && !preact && alpha == 1.f &&
+      aux_mode <= 1 && in_dtype == out_dtype) {
+    SkinnyArgs a;
+    a.x = A; a.ldx = lda; a.M = (int)M; a.K = (int)K; a.dtype = in_dtype;
+    a.w[0] = B; a.bias[0] = bias; a.n[0] = (int)N; a.ldw = ldb;
+    a.out = C; a.ldo = ldc; a.residual = aux; a.act = act & 0xff;
+    if (N < (1ll << 31) && K < (1ll << 31) && skinny_supported(a)) {
+      ProfScope prof(PROF_GEMM, st, 2.0 * (double)M * (double)N * (double)K);
+      return skinny_gemm(a, st);
+    }
+  }
   if (!g_force_simt && gemm_tc_supported(g)) return gemm_tc(g, st);
   return gemm_simt(g, st);
 }
