@@ -372,6 +372,49 @@ int mt_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v_ca
                  int64_t batch, int64_t heads, int64_t n_new, int64_t pos0, int64_t max_len,
                  int64_t head_dim, int dtype, void* stream);
 
+/* ---- whole-model forward without a graph ----------------------------------
+ * The inference branches of GPT2.forward (gpt2_trainer/gpt2.py:352-374) and of
+ * the nanochat GPT (nanochat_trainer/core/nanochat_gpt.py:301-340): embedding,
+ * blocks, final norm and lm_head queued by one call. Activations live in one
+ * scratch buffer taken from the stream-ordered pool for the call.
+ *   block_ptrs  host array [blocks][16] of device pointers (NULL = absent):
+ *               norm1 weight, bias; norm2 weight, bias; q (or the whole per-head
+ *               [q|k|v] projection of the learned-position model), k, v, output,
+ *               up, down projection weights; biases of the last six in that order
+ *   k_cache     host array [blocks] of device pointers, NULL = no cache; rows of
+ *               the new tokens are written from write_pos on (a ring of max_len
+ *               rows); kv_len counts the rows held afterwards, `past` those held
+ *               before (0 = the new tokens are the prompt and attend causally
+ *               among themselves)
+ *   position    index of the first new token in the position / rotary tables
+ *   logits      [batch, new_tokens, vocab], or [batch, vocab] with last_only;
+ *               softcap > 0 applies softcap * tanh(x / softcap) */
+typedef enum { MT_GPT_LEARNED = 0, MT_GPT_ROTARY = 1 } mt_gpt_kind;
+typedef struct {
+  int32_t kind, dtype;
+  int64_t blocks, width, hidden, heads, kv_heads, vocab;
+  const void *wte, *wpe, *lnf_w, *lnf_b, *head_w, *head_b;
+  const float *cos_t, *sin_t;
+  const void* const* block_ptrs;
+  float eps;
+} mt_gpt_model;
+typedef struct {
+  const int32_t* ids;
+  int64_t batch, new_tokens, past, position, write_pos, kv_len, max_len;
+  void* const* k_cache;
+  void* const* v_cache;
+  mt_strides3 cache_strides;
+  void* logits;
+  int32_t last_only;
+  float softcap;
+} mt_gpt_pass;
+int mt_gpt_forward(const mt_gpt_model* model, const mt_gpt_pass* pass, void* stream);
+/* Index of the largest element of each row of x [rows, cols], the first one of equals and the
+ * first NaN if there is one (numpy.argmax, gpt2_trainer/inference_gpt2.py:137-174): written to
+ * idx[row] and, when given, to out[row * ld_out]. */
+int mt_argmax_rows(const void* x, int32_t* idx, int32_t* out, int64_t rows, int64_t cols, int64_t ld_out,
+                   int dtype, void* stream);
+
 /* AdamW.step (mytorch/optim/optimizers.py:342-371), GradScaler.unscale_grads +
  * the inf/nan scan (mytorch/accelerate.py:71-89, 716-729), clip_grad_norm_
  * (mytorch/accelerate.py:799-856) and the master->half copy of

@@ -34,6 +34,20 @@ class TensorList(C.Structure):
                 ("n_tensors", C.c_int64), ("n_chunks", C.c_int64)]
 
 
+class GptModel(C.Structure):
+    _fields_ = ([("kind", C.c_int32), ("dtype", C.c_int32)]
+                + [(n, C.c_int64) for n in ("blocks", "width", "hidden", "heads", "kv_heads", "vocab")]
+                + [(n, C.c_void_p) for n in ("wte", "wpe", "lnf_w", "lnf_b", "head_w", "head_b", "cos_t", "sin_t", "block_ptrs")]
+                + [("eps", C.c_float)])
+
+
+class GptPass(C.Structure):
+    _fields_ = ([("ids", C.c_void_p)]
+                + [(n, C.c_int64) for n in ("batch", "new_tokens", "past", "position", "write_pos", "kv_len", "max_len")]
+                + [("k_cache", C.c_void_p), ("v_cache", C.c_void_p), ("cache_strides", Strides3), ("logits", C.c_void_p),
+                   ("last_only", C.c_int32), ("softcap", C.c_float)])
+
+
 if not os.path.exists(LIB_PATH):
     raise ImportError(
         f"{LIB_PATH} is missing: build it with `python mytorch_b200/csrc/build.py` "
@@ -125,6 +139,8 @@ _SIG = {
     "mt_attn_decode": [_p, _p, _p, _p, _S, _S, _S, _i64, _i64, _i64, _i64, _i64, _f, _i, _i, _p],
     "mt_attn_decode_gqa": [_p, _p, _p, _p, _S, _S, _S, _i64, _i64, _i64, _i64, _i64, _i64, _f, _i, _i, _p],
     "mt_kv_append": [_p, _p, _p, _p, _S, _S, _S, _i64, _i64, _i64, _i64, _i64, _i64, _i, _p],
+    "mt_gpt_forward": [C.POINTER(GptModel), C.POINTER(GptPass), _p],
+    "mt_argmax_rows": [_p, _p, _p, _i64, _i64, _i64, _i, _p],
     "mt_gradnorm_multi": [C.POINTER(TensorList), _i, _p, _p, _p, _p],
     "mt_adamw_multi": [C.POINTER(TensorList), _i, _i, _f, C.c_double, C.c_double, _f, _p, _p, _f, _p, _i, _p, _i, _p],
     "mt_scaler_update": [_p, _p, _f, _f, _i, _f, _i, _p],

@@ -3,15 +3,16 @@ and position embeddings, pre-LayerNorm blocks (attention + GELU MLP, 4x), final
 LayerNorm, lm_head tied to the token embedding. Same config fields, module
 names and state_dict keys, so checkpoints move between the two.
 
-Only the training path is here (no KV cache). The attention module reads the
+The attention module reads the
 per-head interleaved [q|k|v] projection in place (see F.qkv_attention) and the
 embedding pair is one kernel; everything else is the same sequence of ops.
 """
+import ctypes as C
 from dataclasses import dataclass
 
 import numpy as np
 
-from . import _lib, nn
+from . import _lib, infer, nn
 from .array import DeviceArray, stream
 from .nn import functional as F
 from .tensor import Tensor
@@ -51,6 +52,21 @@ class Cache:
 
     def get_seq_len(self, layer_idx=0):
         return min(self._appended[layer_idx], self.max_seq_len)
+
+    def reserve(self, batch, heads, head_dim, dtype):
+        """All layers' rings, allocated together when none of them exists yet. False when the layers
+        do not hold the same number of rows."""
+        if all(k is None for k in self.key_cache):
+            n = len(self.key_cache)
+            rings = DeviceArray.empty((2 * n, batch, heads, self.max_seq_len, head_dim), dtype)
+            ring = lambda i: rings.rows(i, i + 1).reshape(batch, heads, self.max_seq_len, head_dim)
+            self.key_cache = [ring(2 * i) for i in range(n)]
+            self.value_cache = [ring(2 * i + 1) for i in range(n)]
+        elif any(k is None for k in self.key_cache):
+            return False
+        kc = self.key_cache[0]
+        assert kc.shape[0] == batch and kc.dtype == dtype, "cache was created for another batch size or dtype"
+        return all(n == self._appended[0] for n in self._appended)
 
     def update(self, k_ptr, v_ptr, strides, batch, heads, n_new, head_dim, dtype, layer_idx):
         """Appends n_new rows read through (ptr, strides) and returns (keys, values, rows held)."""
@@ -175,6 +191,30 @@ def _init_weights(module):     # gpt2_trainer/gpt2.py:376-389
             nn.init.zeros_(module.bias)
 
 
+def _plan(model):
+    """Describes the model to the library's whole-model forward (see infer.Plan)."""
+    cfg, plain = model.config, infer.plain
+    ok = plain(model, GPT2) and plain(model.embeddings, Embeddings) and plain(model.final_layer_norm, nn.LayerNorm) \
+        and plain(model.lm_head, nn.Linear) and model.lm_head.act_func is None
+    rows = []
+    for b in model.blocks:
+        ok = ok and plain(b, TransformerBlock) and plain(b.attention, Attention) and plain(b.feedforward, FeedForward)
+        if not ok:
+            break
+        a, f = b.attention, b.feedforward
+        linears = (a.qkv_proj, a.out_proj, f.intermediate_dense, f.out_proj)
+        ok = all(plain(m, nn.Linear) for m in linears) and plain(b.layernorm1, nn.LayerNorm) and plain(b.layernorm2, nn.LayerNorm) \
+            and a.proj_drop.p == f.intermediate_dropout.p == f.output_dropout.p == 0.0 \
+            and [m.act_func for m in linears] == [None, None, "gelu", None] and a.num_heads == cfg.num_heads
+        rows.append((b.layernorm1, b.layernorm2, a.qkv_proj, None, None, a.out_proj, f.intermediate_dense, f.out_proj))
+    if not ok:
+        return infer.NoPlan(model.blocks)
+    e = model.embeddings
+    return infer.Plan(model, 0, {"wte": e.char_embeddings, "wpe": e.position_embeddings, "lnf": model.final_layer_norm,
+                                 "head": model.lm_head}, model.blocks, rows, cfg.num_heads, cfg.num_heads,
+                      cfg.embed_dim * cfg.mlp_ratio, cfg.vocab_size)
+
+
 class GPT2(nn.Module):
     def __init__(self, config):
         super().__init__()
@@ -195,9 +235,35 @@ class GPT2(nn.Module):
         activations (gpt2.py:349-365)."""
         self._gradient_checkpointing_enabled = True
 
+    def _planned(self, plan, ids, cache=None, last_only=False):
+        """The whole forward as one library call (no graph); None when the cache's layers differ."""
+        B, T = ids.shape
+        if cache is None:
+            assert T <= self.config.max_seq_len, "position table exhausted"
+            return plan.run(ids, last_only=last_only)
+        cfg, n = self.config, cache.max_seq_len
+        D = plan.head_dim
+        past = cache.get_seq_len()
+        assert past + T <= cfg.max_seq_len, "position table exhausted"
+        if not cache.reserve(B, cfg.num_heads, D, plan.dtype) or T > n or (past and D not in (64, 128)):
+            return None
+        L = len(cache.key_cache)
+        ptrs = C.c_void_p * L
+        out = plan.run(ids, past=past, position=past, write_pos=cache._appended[0] % n, kv_len=min(past + T, n), max_len=n,
+                       k_cache=C.cast(ptrs(*[k.ptr for k in cache.key_cache]), C.c_void_p),
+                       v_cache=C.cast(ptrs(*[v.ptr for v in cache.value_cache]), C.c_void_p),
+                       cache_strides=_lib.Strides3(cfg.num_heads * n * D, n * D, D), last_only=last_only)
+        cache._appended = [a + T for a in cache._appended]
+        return out
+
     def forward(self, x, cache=None):
         """Logits; with a `Cache`, (logits, cache) as in gpt2.py:352-374."""
         from .utils.checkpoint import checkpoint
+        plan = infer.plan_of(self, _plan) if x.data.size else None
+        if plan is not None:
+            out = self._planned(plan, x.data, cache)
+            if out is not None:
+                return Tensor(out) if cache is None else (Tensor(out), cache)
         past_length = cache.get_seq_len() if cache is not None else 0
         x = self.embeddings(x, past_length)
         for layer_idx, block in enumerate(self.blocks):
@@ -211,6 +277,18 @@ class GPT2(nn.Module):
         logits = self.lm_head(x)
         return logits if cache is None else (logits, cache)
 
+    def _generate_greedy(self, plan, ids, cache, n):
+        """The arg-max stays on the device and is the next step's input: the host queues all steps
+        and reads the ids back once."""
+        out = DeviceArray.empty((ids.shape[0], n), "int32")
+        feed = Tensor(ids).data
+        for i in range(n):
+            logits = self._planned(plan, feed, cache, last_only=True)
+            if logits is None:
+                return None
+            feed = infer.greedy(logits, out, i)
+        return out.numpy()
+
     def generate(self, input_ids, max_new_tokens, temperature=1.0, top_k=None, use_cache=True, seed=None):
         """Autoregressive sampling as in gpt2_trainer/inference_gpt2.py:137-174: the prompt fills
         the cache, then one token per step; temperature-scaled softmax (optionally restricted to
@@ -221,9 +299,16 @@ class GPT2(nn.Module):
         cache = Cache(self.config) if use_cache else None
         feed = ids
         with no_grad():
+            plan = infer.plan_of(self, _plan)
+            if plan is not None and temperature == 0 and use_cache and max_new_tokens > 0 and ids.size:
+                new = self._generate_greedy(plan, ids, cache, max_new_tokens)
+                if new is not None:
+                    return np.concatenate([ids, new], axis=1)
             for _ in range(max_new_tokens):
-                out = self.forward(Tensor(feed), cache=cache)
-                logits = out[0] if use_cache else out
+                logits = self._planned(plan, Tensor(feed).data, cache, last_only=True) if plan is not None else None
+                if logits is None:
+                    out = self.forward(Tensor(feed), cache=cache)
+                    logits = out[0] if use_cache else out
                 last = logits.numpy()[:, -1, :].astype(np.float64)
                 if temperature == 0:
                     nxt = last.argmax(-1)

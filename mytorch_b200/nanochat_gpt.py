@@ -14,12 +14,13 @@ Unlike the reference's training dispatcher, which drops `softcap` before the
 loss is computed (mytorch/nn/functional/losses/cross_entropy.py:178), the cap
 is applied, as the model definition intends.
 """
+import ctypes as C
 import math
 from dataclasses import dataclass
 
 import numpy as np
 
-from . import _lib, nn
+from . import _lib, infer, nn
 from .array import DeviceArray, stream
 from .nn import functional as F
 from .tensor import Tensor
@@ -41,6 +42,15 @@ class KVCache:
 
     def reset(self):
         self._pos = 0
+
+    def layers(self, dtype):
+        """(keys, values) as host arrays of one device pointer per layer."""
+        if self.k_cache is None:
+            self.k_cache = DeviceArray.empty(self.cache_shape, dtype)
+            self.v_cache = DeviceArray.empty(self.cache_shape, dtype)
+        n, step = self.cache_shape[0], self.k_cache.nbytes // max(1, self.cache_shape[0])
+        ptrs = C.c_void_p * n
+        return tuple(C.cast(ptrs(*[c.ptr + i * step for i in range(n)]), C.c_void_p) for c in (self.k_cache, self.v_cache))
 
     def update(self, k_ptr, v_ptr, strides, n_new, dtype, layer_idx):
         L, B, H, S, D = self.cache_shape
@@ -167,6 +177,28 @@ def _init_weights(module):      # nanochat_gpt.py:352-369
         nn.init.normal_(module.weight, mean=0.0, std=0.02)
 
 
+def _plan(model):
+    """Describes the model to the library's whole-model forward (see infer.Plan)."""
+    cfg, plain = model.config, infer.plain
+    D = cfg.embed_dim // cfg.num_q_heads
+    ok = plain(model, GPT) and plain(model.embeddings, Embeddings) and plain(model.embeddings.embeddings, nn.Embedding) \
+        and plain(model.lm_head, nn.Linear) and model.lm_head.act_func is None and D in (64, 128)
+    rows = []
+    for b in model.blocks:
+        ok = ok and plain(b, TransformerBlock) and plain(b.attention, Attention) and plain(b.feedforward, FeedForward)
+        if not ok:
+            break
+        a, f = b.attention, b.feedforward
+        linears = (a.q_proj, a.k_proj, a.v_proj, a.out_proj, f.intermediate_dense, f.out_proj)
+        ok = all(plain(m, nn.Linear) for m in linears) and [m.act_func for m in linears] == [None] * 4 + ["relu_squared", None] \
+            and (a.num_heads, a.num_kv_heads) == (cfg.num_q_heads, cfg.num_kv_heads)
+        rows.append((None, None, a.q_proj, a.k_proj, a.v_proj, a.out_proj, f.intermediate_dense, f.out_proj))
+    if not ok:
+        return infer.NoPlan(model.blocks)
+    return infer.Plan(model, 1, {"wte": model.embeddings.embeddings, "head": model.lm_head}, model.blocks, rows, cfg.num_q_heads,
+                      cfg.num_kv_heads, cfg.embed_dim * cfg.mlp_ratio, cfg.vocab_size, model.cos, model.sin)
+
+
 class GPT(nn.Module):
     def __init__(self, config):
         super().__init__()
@@ -193,8 +225,34 @@ class GPT(nn.Module):
         """Recompute each block in the backward pass (nanochat_gpt.py:318-322)."""
         self._gradient_checkpointing_enabled = True
 
+    def _planned(self, plan, ids, cache=None, last_only=False):
+        """The whole forward as one library call (no graph, soft-capped outside training); None when
+        the cache has another shape than this model's."""
+        cfg = self.config
+        B, T = ids.shape
+        past = cache.pos if cache is not None else 0
+        assert past + T <= cfg.max_seq_len, "sequence longer than the rotary table"
+        cap = float(cfg.softcap or 0.0) if not self.training else 0.0
+        if cache is None:
+            return plan.run(ids, last_only=last_only, softcap=cap)
+        L, Bc, Hk, S, D = cache.cache_shape
+        if (L, Bc, Hk, D) != (cfg.num_blocks, B, cfg.num_kv_heads, plan.head_dim) or (past and D not in (64, 128)) \
+                or (cache.k_cache is not None and cache.k_cache.dtype != plan.dtype):
+            return None
+        assert past + T <= S, "You have filled up your Cache!"
+        k, v = cache.layers(plan.dtype)
+        out = plan.run(ids, past=past, position=past, write_pos=past, kv_len=past + T, max_len=S, k_cache=k, v_cache=v,
+                       cache_strides=_lib.Strides3(Hk * S * D, S * D, D), last_only=last_only, softcap=cap)
+        cache._pos += T
+        return out
+
     def forward(self, input_ids, target_ids=None, cache=None):
         B, T = input_ids.shape
+        plan = infer.plan_of(self, _plan) if target_ids is None and B * T else None
+        if plan is not None:
+            out = self._planned(plan, input_ids.data, cache)
+            if out is not None:
+                return (Tensor(out),) if cache is None else (Tensor(out), cache)
         past = cache.pos if cache is not None else 0
         assert past + T <= self.config.max_seq_len, "sequence longer than the rotary table"
         cos, sin = self.cos.rows(past, past + T), self.sin.rows(past, past + T)   # positions continue after the cache
@@ -236,8 +294,19 @@ class GPT(nn.Module):
         self.eval()
         feed = ids
         with no_grad():
+            plan = infer.plan_of(self, _plan) if ids.size and max_new_tokens > 0 else None
+            if plan is not None and temperature == 0:
+                # the arg-max stays on the device and is the next step's input; one read at the end
+                out, dev = DeviceArray.empty((ids.shape[0], max_new_tokens), "int32"), Tensor(ids).data
+                for i in range(max_new_tokens):
+                    dev = infer.greedy(self._planned(plan, dev, cache, last_only=True), out, i)
+                ids = np.concatenate([ids, out.numpy()], axis=1)
+                max_new_tokens = 0
             for _ in range(max_new_tokens):
-                logits, cache = self.forward(Tensor(feed), None, cache=cache)
+                if plan is not None:
+                    logits = self._planned(plan, Tensor(feed).data, cache, last_only=True)
+                else:
+                    logits, cache = self.forward(Tensor(feed), None, cache=cache)
                 last = logits.numpy()[:, -1, :].astype(np.float64)
                 if temperature == 0:
                     nxt = last.argmax(-1)
