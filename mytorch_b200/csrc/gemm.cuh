@@ -46,6 +46,8 @@ __device__ __forceinline__ float act_grad(float x, int act) {
   }
 }
 int gemm_simt(const GemmArgs& g, cudaStream_t st);
+bool gemm_split_supported(const GemmArgs& g);      // fp32, and half operands that gemm_tc cannot address
+int gemm_split(const GemmArgs& g, cudaStream_t st);
 bool gemm_tc_supported(const GemmArgs& g);
 int gemm_tc(const GemmArgs& g, cudaStream_t st);
 }  // namespace mt

@@ -1,0 +1,497 @@
+// Tensor-core GEMM for operands that gemm_tcgen05.cu does not take, with sums at least as exact as a
+// chain of fp32 FMAs: fp32 matrices, and half matrices whose pointers or pitches TMA cannot address.
+//
+// Two launches. `prepare_kernel` rewrites the operands with a 16-byte pitch: an fp32 value x becomes three
+// bf16 planes h + m + l = x (8 significant bits each, rounded to nearest, so what is left over is
+// below 2^-26 |x|), a half value is copied. `gemm_split_kernel` then multiplies plane by plane:
+//   fp32: l.h + h.l + m.m + m.h + h.m + h.h, smallest first; the products left out (m.l, l.m, l.l) are below
+//   2^-25 of a term. Every bf16 product is exact in the fp32 accumulator.
+// The accumulator in tensor memory is not kept over all of K: after each chunk of K the epilogue warps
+// add it to fp32 registers (round to nearest) while the next chunk goes to the other accumulator.
+// Relative error against 64 bits (2-norm, normal data): K = 256 8.6e-8 (FMA chain 2.9e-7), 768 1.0e-7 (5.0e-7),
+// 4096 1.1e-7 (1.1e-6), 8192 2.2e-7 (1.6e-6).
+//
+// One 128 x 128 tile per CTA (persistent): a slot of the ring holds one plane of A and of B (2 x 16 KB); the
+// 24 MMAs of a 64-deep slice (1536 tensor cycles) read 96 KB, 64 B per clock and SM. Where tiles are few
+// (weight gradients of small layers), K is split over a cluster of up to eight CTAs whose sums meet
+// through distributed shared memory in a fixed order: no atomics, the same bits every time.
+// fp32: 8192 x 768 -> 3072 1414 -> 369 us, its weight gradient 1529 -> 258, 4096 x 256 -> 1024 102 -> 47, 256 x 4096 x 256
+// 209 -> 25; bf16 with odd pitches: 3885 x 50257 -> 768 15158 -> 719 us, 50257 x 3885 -> 768 12345 -> 658.
+//
+// A result that is not finite (an operand is, or |x| > 3.39e38 rounds to bf16 infinity) is computed
+// again as a plain fp32 dot product, so infinities and NaNs come out as fp32 arithmetic gives them.
+// Operands below 2^-108 lose their last plane to bf16's exponent range.
+#include "gemm.cuh"
+#include "sm100.cuh"
+#include "prof.cuh"
+#include "tempbuf.cuh"
+#include <atomic>
+#include <string.h>
+
+namespace mt {
+
+using namespace sm100;
+
+constexpr int kSpM = 128, kSpN = 128, kSpK = 64;
+constexpr int kSpPlane = 128 * kSpK * 2;             // 16 KB: one plane of one operand's tile
+constexpr int kSpSlot = 2 * kSpPlane;
+constexpr int kSpSlots = 6;
+constexpr int kSpEpiWarps = 8;
+constexpr int kSpThreads = 64 + 32 * kSpEpiWarps;
+constexpr int kSpStage = 32 * 33 * 4;                // an epilogue warp's 32 x 32 transpose buffer
+constexpr int kSpSmem = kSpSlots * kSpSlot + kSpEpiWarps * kSpStage + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int kSpPitch = kSpN + 1;                   // row pitch (floats) of the sums a cluster exchanges
+static_assert(kSpM * kSpPitch * 4 <= kSpSlots * kSpSlot, "a tile's sums fit the ring");
+
+struct SplitParams {
+  const void* A; const void* B; void* C; void* preact; const void* bias; const void* aux;
+  int64_t M, N, K, lda, ldb, ldc;
+  int trans_a, trans_b, in_dtype, out_dtype, act, aux_mode, accumulate;
+  float alpha;
+  int tiles_m, tiles_n, n_fast, csize, kb_total, kb_per_rank, chunk;
+  int* flag;
+};
+
+__device__ __forceinline__ float load_typed(const void* p, int64_t i, int dt) {
+  return dt == MT_F32 ? ((const float*)p)[i] : dt == MT_F16 ? __half2float(((const __half*)p)[i]) : __bfloat162float(((const __nv_bfloat16*)p)[i]);
+}
+__device__ __forceinline__ void store_typed(void* p, int64_t i, int dt, float v) {
+  if (dt == MT_F32) ((float*)p)[i] = v;
+  else if (dt == MT_F16) ((__half*)p)[i] = __float2half_rn(v);
+  else ((__nv_bfloat16*)p)[i] = __float2bfloat16_rn(v);
+}
+
+// The dot product of one output in plain fp32.
+static __device__ __noinline__ float split_dot(const SplitParams& P, int64_t m, int64_t n) {
+  const float* a = (const float*)P.A + (P.trans_a ? m : m * P.lda);
+  const float* b = (const float*)P.B + (P.trans_b ? n * P.ldb : n);
+  const int64_t sa = P.trans_a ? P.lda : 1, sb = P.trans_b ? 1 : P.ldb;
+  float v = 0.f;
+  for (int64_t k = 0; k < P.K; ++k) v = fmaf(a[k * sa], b[k * sb], v);
+  return v;
+}
+
+// Everything behind the sum of one output; aux and old are what its aux operand and C hold (0 where not read).
+template <bool F32>
+__device__ __forceinline__ void split_finish(const SplitParams& P, float v, float bias, float aux, float old, int64_t m, int64_t n) {
+  if (F32 && !(fabsf(v) <= 3.402823466e38f)) v = split_dot(P, m, n);
+  v = P.alpha * v + bias;
+  const int64_t off = m * P.ldc + n;
+  if (P.preact) store_typed(P.preact, off, P.out_dtype, (P.act & kActStoreGrad) ? act_grad(v, P.act) : v);
+  switch (P.act & 0xff) {
+    case MT_ACT_GELU: v = 0.5f * v * (1.f + tanhf(0.7978845608f * (v + 0.044715f * v * v * v))); break;
+    case MT_ACT_RELU2: { const float r = fmaxf(v, 0.f); v = r * r; break; }
+    case MT_ACT_RELU: v = fmaxf(v, 0.f); break;
+    default: break;
+  }
+  if (P.aux_mode) v = aux_apply(v, aux, P.aux_mode);
+  if (P.accumulate) v += old;
+  store_typed(P.C, off, P.out_dtype, v);
+}
+
+template <bool F32, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kSpThreads, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitParams P) {
+  constexpr int PLANES = F32 ? 3 : 1;
+  extern __shared__ uint8_t sp_smem[];
+  const uint32_t raw = smem_u32(sp_smem);
+  const uint32_t base = (raw + 1023u) & ~1023u;      // the 128-byte swizzle repeats every 1024 bytes
+  uint8_t* const base_ptr = sp_smem + (base - raw);
+  float* const stages = reinterpret_cast<float*>(base_ptr + kSpSlots * kSpSlot);
+  uint8_t* const bar_ptr = base_ptr + kSpSlots * kSpSlot + kSpEpiWarps * kSpStage;
+  const uint32_t bar0 = smem_u32(bar_ptr);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (kSpSlots + s); };
+  auto accf_bar = [&](int b) { return bar0 + 8u * (2 * kSpSlots + b); };
+  auto acce_bar = [&](int b) { return bar0 + 8u * (2 * kSpSlots + 2 + b); };
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bar_ptr + 8 * (2 * kSpSlots + 4));
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int csize = P.csize;
+  const int rank = csize > 1 ? (int)cluster_ctarank() : 0;
+  const int worker = (int)blockIdx.x / csize, workers = (int)gridDim.x / csize;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSpSlots; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), kSpEpiWarps); }
+    *abort_flag = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 2 * kSpN); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  griddep_launch();
+  griddep_wait();
+
+  const int total = P.tiles_m * P.tiles_n;
+  const int kb0 = rank * P.kb_per_rank, kb1 = min(P.kb_total, kb0 + P.kb_per_rank);
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer --
+    if (lane == 0) {
+      prefetch_tmap(&tmA);
+      prefetch_tmap(&tmB);
+      int slot = 0;
+      uint32_t phase = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (int t = worker; t < total && ok; t += workers) {
+        const int m0 = (P.n_fast ? t / P.tiles_n : t % P.tiles_m) * kSpM, n0 = (P.n_fast ? t % P.tiles_n : t / P.tiles_m) * kSpN;
+        for (int kb = kb0; kb < kb1 && ok; ++kb) {
+          for (int pl = 0; pl < PLANES; ++pl) {
+            if (!mbar_wait(empty_bar(slot), phase ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t sa = base + slot * kSpSlot, sb = sa + kSpPlane, bar = full_bar(slot);
+            mbar_expect_tx(bar, kSpSlot);
+            if (!A_MN) tma_load_3d(sa, &tmA, bar, kb * kSpK, m0, pl);
+            else for (int j = 0; j < 2; ++j) tma_load_3d(sa + j * (kSpK * 128), &tmA, bar, m0 + j * 64, kb * kSpK, pl);
+            if (!B_MN) tma_load_3d(sb, &tmB, bar, kb * kSpK, n0, pl);
+            else for (int j = 0; j < 2; ++j) tma_load_3d(sb + j * (kSpK * 128), &tmB, bar, n0 + j * 64, kb * kSpK, pl);
+            ++issued;
+            if (++slot == kSpSlots) { slot = 0; phase ^= 1u; }
+          }
+        }
+      }
+      if (!ok) {                                       // bounded: the copies in flight land before shared memory goes away
+        const long long n = issued < kSpSlots ? issued : kSpSlots;
+        int s = slot;
+        uint32_t ph = phase;
+        for (long long i = 0; i < n; ++i) {
+          if (--s < 0) { s = kSpSlots - 1; ph ^= 1u; }
+          const long long t0 = clock64();
+          while (!mbar_try_wait(full_bar(s), ph) && clock64() - t0 < kWaitLimitCycles) {}
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------- MMA issuer --
+    if (lane == 0) {
+      const uint32_t idesc = idesc_f16(F32 || P.in_dtype == MT_BF16, A_MN, B_MN, kSpM, kSpN);
+      int slot = 0, it = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = worker; t < total && ok; t += workers) {
+        for (int kc = kb0; kc < kb1 && ok; kc += P.chunk, ++it) {
+          const int buf = it & 1;
+          if (!mbar_wait(acce_bar(buf), ((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t d = tmem_base + buf * kSpN;
+          const int ke = min(kb1, kc + P.chunk);
+          for (int kb = kc; kb < ke && ok; ++kb) {
+            // the slots of a slice are neighbours: kSpSlots is a multiple of PLANES
+            for (int pl = 0; pl < PLANES && ok; ++pl) ok = mbar_wait(full_bar(slot + pl), phase, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            auto product = [&](int pa, int pb, uint32_t acc) {
+              const uint32_t sa = base + (slot + pa) * kSpSlot, sb = base + (slot + pb) * kSpSlot + kSpPlane;
+              uint64_t a[4], b[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                a[k] = A_MN ? smem_desc_sw128(sa + k * 2048, kSpK * 128, 1024) : smem_desc_sw128(sa + k * 32, 16, 1024);
+                b[k] = B_MN ? smem_desc_sw128(sb + k * 2048, kSpK * 128, 1024) : smem_desc_sw128(sb + k * 32, 16, 1024);
+              }
+              umma_f16_x4(d, a, b, idesc, acc);
+            };
+            const uint32_t acc = kb > kc ? 1u : 0u;
+            if (F32) {
+              product(2, 0, acc);
+              product(0, 2, 1u);
+              product(1, 1, 1u);
+              product(1, 0, 1u);
+              product(0, 1, 1u);
+              product(0, 0, 1u);
+            } else {
+              product(0, 0, acc);
+            }
+            for (int pl = 0; pl < PLANES; ++pl) umma_commit(empty_bar(slot + pl));
+            slot += PLANES;
+            if (slot == kSpSlots) { slot = 0; phase ^= 1u; }
+          }
+          if (ok) umma_commit(accf_bar(buf));
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue --
+    const int quarter = warp & 3, c0 = ((warp - 2) >> 2) * (kSpN / 2);      // 32 rows, 64 columns of the tile
+    float* const stage = stages + (warp - 2) * (32 * 33);
+    int it = 0;
+    bool ok = true;
+    for (int t = worker; t < total && ok; t += workers) {
+      const int64_t m0 = (int64_t)(P.n_fast ? t / P.tiles_n : t % P.tiles_m) * kSpM + quarter * 32;
+      const int64_t n0 = (int64_t)(P.n_fast ? t % P.tiles_n : t / P.tiles_m) * kSpN + c0;
+      float acc[64];
+#pragma unroll
+      for (int e = 0; e < 64; ++e) acc[e] = 0.f;
+      for (int kc = kb0; kc < kb1; kc += P.chunk, ++it) {
+        const int buf = it & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(accf_bar(buf), (it >> 1) & 1, abort_flag))) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * kSpN + c0;
+        uint32_t r[64];
+        tmem_ld32(taddr, r);
+        tmem_ld32(taddr + 32, r + 32);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acce_bar(buf));
+#pragma unroll
+        for (int e = 0; e < 64; ++e) acc[e] += __uint_as_float(r[e]);
+      }
+      if (!ok) break;
+      if (csize > 1) {
+        // all copies and MMAs of this CTA are done: its ring holds the sums for the cluster
+        float* rows = reinterpret_cast<float*>(base_ptr) + (quarter * 32 + lane) * kSpPitch + c0;
+#pragma unroll
+        for (int e = 0; e < 64; ++e) rows[e] = acc[e];
+      } else {
+        // thread = row becomes lane = column: rows of 128 bytes to and from global memory, any pitch
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int64_t n = n0 + h * 32 + lane;
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = acc[h * 32 + e];
+          __syncwarp();
+          if (n < P.N) {
+            const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
+            const int rows = (int)min((int64_t)32, P.M - m0);
+            for (int r0 = 0; r0 < rows; r0 += 8) {            // eight rows' reads in flight at a time
+              float v[8], aux[8], old[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const int64_t off = (m0 + min(r0 + u, rows - 1)) * P.ldc + n;
+                v[u] = stage[(r0 + u) * 33 + lane];
+                aux[u] = P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f;
+                old[u] = P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f;
+              }
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                if (r0 + u < rows) split_finish<F32>(P, v[u], bias, aux[u], old[u], m0 + r0 + u, n);
+            }
+          }
+        }
+      }
+    }
+  }
+
+  // ------------------------------------------------- sums of a cluster, teardown --
+  tc_fence_before();
+  __syncthreads();
+  if (csize > 1) {
+    cluster_sync_all();
+    if (worker < total) {
+      const int64_t m0 = (int64_t)(P.n_fast ? worker / P.tiles_n : worker % P.tiles_m) * kSpM;
+      const int64_t n0 = (int64_t)(P.n_fast ? worker % P.tiles_n : worker / P.tiles_m) * kSpN;
+      const int share = kSpM / csize;
+      float bias[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t n = n0 + j * 32 + lane;
+        bias[j] = P.bias && n < P.N ? load_typed(P.bias, n, P.in_dtype) : 0.f;
+      }
+      for (int r = rank * share + warp; r < (rank + 1) * share && m0 + r < P.M; r += kSpThreads / 32) {
+        float v[4] = {}, aux[4] = {}, old[4] = {};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int64_t n = n0 + j * 32 + lane, off = (m0 + r) * P.ldc + n;
+          if (n < P.N && P.aux_mode) aux[j] = load_typed(P.aux, off, P.out_dtype);
+          if (n < P.N && P.accumulate) old[j] = load_typed(P.C, off, P.out_dtype);
+        }
+        for (int c = 0; c < csize; ++c) {
+          const uint32_t src = mapa_shared(base + (uint32_t)(r * kSpPitch + lane) * 4u, (uint32_t)c);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float x;
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(src + 128u * j) : "memory");
+            v[j] += x;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int64_t n = n0 + j * 32 + lane;
+          if (n < P.N) split_finish<F32>(P, v[j], bias[j], aux[j], old[j], m0 + r, n);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();                                // nobody leaves while its sums are still being read
+  }
+  if (threadIdx.x == 0 && *abort_flag && P.flag) atomicMax(P.flag, 106);   // a bounded wait expired
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 2 * kSpN);
+  }
+}
+
+// One operand [rows, cols] (row stride ld) and where its planes go: [planes][rows][pitch], pitch a multiple of 8.
+struct PrepareJob { const void* src; void* dst; int64_t rows, cols, ld, pitch, units; int vec; };
+
+// A thread rewrites eight neighbouring values. HBM-bound: fp32 reads 4 and writes 6 bytes a value.
+template <bool F32>
+__global__ void __launch_bounds__(256)
+prepare_kernel(const PrepareJob a, const PrepareJob b) {
+  grid_dependency_wait();
+  allow_dependents();
+  const int64_t total = a.units + b.units;
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (int64_t)gridDim.x * blockDim.x) {
+    const bool first = u < a.units;
+    const PrepareJob& j = first ? a : b;
+    const int64_t i = first ? u : u - a.units;
+    const int64_t per_row = j.pitch / 8;
+    const int64_t row = total < (1ll << 32) ? (int64_t)((uint32_t)i / (uint32_t)per_row) : i / per_row;
+    const int64_t col = (i - row * per_row) * 8;
+    const int64_t dst = row * j.pitch + col;
+    if (F32) {
+      const float* s = (const float*)j.src + row * j.ld + col;
+      float x[8];
+      if (j.vec && col + 8 <= j.cols) {
+        const float4 p = *reinterpret_cast<const float4*>(s), q = *reinterpret_cast<const float4*>(s + 4);
+        x[0] = p.x; x[1] = p.y; x[2] = p.z; x[3] = p.w;
+        x[4] = q.x; x[5] = q.y; x[6] = q.z; x[7] = q.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = col + e < j.cols ? s[e] : 0.f;
+      }
+      Vec16<__nv_bfloat16> h, m, l;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        h.e[e] = __float2bfloat16_rn(x[e]);
+        const float r = x[e] - __bfloat162float(h.e[e]);       // exact
+        m.e[e] = __float2bfloat16_rn(r);
+        l.e[e] = __float2bfloat16_rn(r - __bfloat162float(m.e[e]));
+      }
+      __nv_bfloat16* d = (__nv_bfloat16*)j.dst + dst;
+      const int64_t plane = j.rows * j.pitch;
+      h.store(d);
+      m.store(d + plane);
+      l.store(d + 2 * plane);
+    } else {
+      const uint16_t* s = (const uint16_t*)j.src + row * j.ld + col;
+      __align__(16) uint16_t x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = col + e < j.cols ? s[e] : (uint16_t)0;
+      *reinterpret_cast<uint4*>((uint16_t*)j.dst + dst) = *reinterpret_cast<const uint4*>(x);
+    }
+  }
+}
+
+// The CUDA-core kernel takes about 8 us and 0.05 us per k for each 64 x 64 tile an SM has (measured in fp32: 256^3
+// 21 us, 4096 x 256 x 256 29, 4096 x 256 x 65 15, 4096 x 1024 x 256 102); this path 15-23 us for small products, most of
+// it the host's two launches, allocation and tensor maps (256^3 17 us, 4096 x 256 x 256 20, 4096 x 256 x 65 23).
+constexpr double kSplitMinUs = 24.0;
+
+bool gemm_split_supported(const GemmArgs& g) {
+  if (g.M < 16 || g.N < 16 || g.K < 16) return false;
+  if (g.M >= (1ll << 30) || g.N >= (1ll << 30) || g.K > (1ll << 17)) return false;   // (K: the time a row of plain dot products may take)
+  const double tiles = (double)((g.M + 63) / 64) * (double)((g.N + 63) / 64) / (0.87 * sm_count());
+  return 8.0 + 0.05 * (double)g.K * (tiles > 1.0 ? tiles : 1.0) >= kSplitMinUs;
+}
+
+template <bool F32, bool A_MN, bool B_MN>
+static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const SplitParams& P, int grid, cudaStream_t st) {
+  auto kern = gemm_split_kernel<F32, A_MN, B_MN>;
+  static std::atomic<bool> ready[16];      // per device; racing first calls set the same attribute twice, harmlessly
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16 || !ready[dev].load(std::memory_order_acquire)) {
+    MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpSmem));
+    if (dev >= 0 && dev < 16) ready[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kSpThreads);
+  cfg.dynamicSmemBytes = kSpSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)P.csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap_launches() ? 2 : 1;
+  MT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, P));
+  count_launch();
+  return MT_OK;
+}
+
+int gemm_split(const GemmArgs& g, cudaStream_t st) {
+  const bool f32 = g.in_dtype == MT_F32;
+  const int planes = f32 ? 3 : 1;
+  PrepareJob job[2] = {};
+  const void* src[2] = {g.A, g.B};
+  const int64_t rows[2] = {g.trans_a ? g.K : g.M, g.trans_b ? g.N : g.K};
+  const int64_t cols[2] = {g.trans_a ? g.M : g.K, g.trans_b ? g.K : g.N};
+  const int64_t ld[2] = {g.lda, g.ldb};
+  size_t bytes = 0, at[2] = {0, 0};
+  for (int i = 0; i < 2; ++i) {
+    PrepareJob& j = job[i];
+    j.src = src[i]; j.rows = rows[i]; j.cols = cols[i]; j.ld = ld[i];
+    j.vec = aligned16(src[i]) && ld[i] % 4 == 0;
+    j.pitch = (cols[i] + 7) / 8 * 8;
+    if (!f32 && aligned16(src[i]) && ld[i] % 8 == 0) continue;       // this half operand can be read where it is
+    j.units = rows[i] * (j.pitch / 8);
+    at[i] = bytes;
+    bytes += ((size_t)planes * rows[i] * j.pitch * 2 + 255) / 256 * 256;
+  }
+  ProfScope prof(PROF_GEMM, st, 2.0 * (double)g.M * (double)g.N * (double)g.K);
+  TempBuf tmp(bytes, st);
+  if (!tmp.ok()) {                                                   // no room for the planes
+    cudaGetLastError();
+    return gemm_simt(g, st);
+  }
+  for (int i = 0; i < 2; ++i) job[i].dst = job[i].units ? (char*)tmp.ptr + at[i] : nullptr;
+  const int64_t units = job[0].units + job[1].units;
+  if (units) {
+    const int64_t want = (units + 255) / 256, most = (int64_t)sm_count() * 16;
+    const dim3 grid((unsigned)(want < most ? want : most));
+    if (f32) MT_CHECK_CUDA(launch_overlapped(prepare_kernel<true>, grid, dim3(256), 0, st, job[0], job[1]));
+    else MT_CHECK_CUDA(launch_overlapped(prepare_kernel<false>, grid, dim3(256), 0, st, job[0], job[1]));
+    count_launch();
+  }
+  CUtensorMap map[2];
+  const bool mn[2] = {g.trans_a != 0, g.trans_b == 0};
+  for (int i = 0; i < 2; ++i) {
+    const PrepareJob& j = job[i];
+    const uint64_t pitch = (uint64_t)(j.units ? j.pitch : j.ld);
+    const uint64_t dims[3] = {(uint64_t)j.cols, (uint64_t)j.rows, (uint64_t)planes};
+    const uint64_t strides[2] = {pitch, pitch * (uint64_t)j.rows};
+    const uint32_t box[3] = {64, (uint32_t)(mn[i] ? kSpK : 128), 1};
+    const int rc = make_tmap_nd(&map[i], j.units ? j.dst : j.src, f32 || g.in_dtype == MT_BF16, 3, dims, strides, box);
+    if (rc) return rc;
+  }
+  SplitParams P{};
+  P.A = g.A; P.B = g.B; P.C = g.C; P.preact = g.preact; P.bias = g.bias; P.aux = g.aux;
+  P.M = g.M; P.N = g.N; P.K = g.K; P.lda = g.lda; P.ldb = g.ldb; P.ldc = g.ldc;
+  P.trans_a = g.trans_a; P.trans_b = g.trans_b; P.in_dtype = g.in_dtype; P.out_dtype = g.out_dtype;
+  P.act = g.act; P.aux_mode = g.aux_mode; P.accumulate = g.accumulate; P.alpha = g.alpha;
+  P.tiles_m = (int)((g.M + kSpM - 1) / kSpM);
+  P.tiles_n = (int)((g.N + kSpN - 1) / kSpN);
+  P.kb_total = (int)((g.K + kSpK - 1) / kSpK);
+  P.chunk = f32 || g.out_dtype == MT_F32 ? 1 : 4;      // a half output's own rounding hides what four slices lose
+  P.flag = device_flag_ptr();
+  // Neighbouring tiles share the larger operand's panel unless it fits the L2 anyway.
+  P.n_fast = g.M > g.N ? 1 : 0;
+  const int sms = sm_count();
+  const long long tiles = (long long)P.tiles_m * P.tiles_n;
+  // K over a cluster while that leaves no CTA waiting for an SM and each at least two slices.
+  P.csize = 1;
+  while (P.csize < 8 && tiles * P.csize * 2 <= sms && P.kb_total >= 4 * P.csize) P.csize *= 2;
+  P.kb_per_rank = (P.kb_total + P.csize - 1) / P.csize;
+  while (P.csize > 1 && (P.csize - 1) * P.kb_per_rank >= P.kb_total) {        // no rank without work
+    P.csize /= 2;
+    P.kb_per_rank = (P.kb_total + P.csize - 1) / P.csize;
+  }
+  const int grid = P.csize > 1 ? (int)tiles * P.csize : (int)(tiles < sms ? tiles : sms);
+#define MT_SPLIT(F)                                                                       \
+  (mn[0] ? (mn[1] ? launch_split<F, true, true>(map[0], map[1], P, grid, st)              \
+                  : launch_split<F, true, false>(map[0], map[1], P, grid, st))            \
+         : (mn[1] ? launch_split<F, false, true>(map[0], map[1], P, grid, st)             \
+                  : launch_split<F, false, false>(map[0], map[1], P, grid, st)))
+  return f32 ? MT_SPLIT(true) : MT_SPLIT(false);
+#undef MT_SPLIT
+}
+
+}  // namespace mt

@@ -1039,6 +1039,7 @@ int mt_gemm_ex(const void* A, const void* B, void* C, void* preact, const void* 
     }
   }
   if (!g_force_simt && gemm_tc_supported(g)) return gemm_tc(g, st);
+  if (!g_force_simt && gemm_split_supported(g)) return gemm_split(g, st);
   return gemm_simt(g, st);
 }
 
