@@ -181,8 +181,6 @@ template <> __device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&c)[
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-
-
 // Rows of W in a group (8 in half types, 4 in fp32).
 template <typename T> struct SkinnyGroup { static constexpr int rows = sizeof(T) == 2 ? 8 : 4; };
 
@@ -542,12 +540,6 @@ int skinny_gemm(const SkinnyArgs& a, cudaStream_t st) {
   p.act = a.act; p.softcap = a.softcap;
   p.gamma = a.gamma; p.beta = a.beta; p.eps = a.eps;
   p.early = a.early_weights;
-  p.norm = a.norm;
-  p.flag = device_flag_ptr();
-  p.norm = a.norm;
-  p.flag = device_flag_ptr();
-  p.norm = a.norm;
-  p.flag = device_flag_ptr();
   p.norm = a.norm;
   p.flag = device_flag_ptr();
   if (a.dtype != MT_F32) {

@@ -59,7 +59,7 @@ template <int BN, bool PAIR = false> struct GemmCfg {
 struct GemmParams {
   void* C; void* preact; const void* bias; const void* aux; int aux_mode;
   int64_t M, N, K, ldc;
-  int out_dtype, in_bf16, act, accumulate, vec_store, tma_store;
+  int out_dtype, in_bf16, act, accumulate, tma_store;
   float alpha;
   int tiles_m, tiles_n, splits, kb_per_split, kb_total;
   int stages;   // pipeline stages in use: Cfg::kStages, or one less with the last stage's memory as second staging buffers
@@ -149,41 +149,42 @@ __device__ __forceinline__ float act_apply_tc(float x, int act) {
   }
 }
 
-// Writes 8 consecutive outputs of one row.
+// A 32 x 32 piece of the accumulator (thread = row) to an output that a tensor map cannot describe (odd
+// pitch or address, read-modify-write of a half output): turned in shared memory so that a warp reads and
+// writes 32 neighbouring columns of a row, eight rows at a time. One row per thread wrote single values to 32 rows at
+// once: bf16 3885 x 768 -> 50257 2.2 ms, 0.83 now.
 template <typename TO>
-__device__ __forceinline__ void store8(TO* p, const float* v, int n_valid, bool vec, int accumulate) {
-  if (vec && n_valid == 8) {
-    if (sizeof(TO) == 2) {
-      __align__(16) TO o[8];
-      if (accumulate) {
-        *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void epilogue_rows(const GemmParams& P, const uint32_t (&r)[32], float* stage, int lane, int64_t m0, int rows,
+                                              int64_t n, bool add_bias) {
+  __syncwarp();
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = from_f<TO>(to_f(o[e]) + v[e]);
-      } else {
+  for (int e = 0; e < 32; ++e) stage[lane * 32 + (e ^ lane)] = __uint_as_float(r[e]);
+  __syncwarp();
+  if (n >= P.N) return;
+  TO* const C = reinterpret_cast<TO*>(P.C);
+  TO* const pre = reinterpret_cast<TO*>(P.preact);
+  const TO* const aux = reinterpret_cast<const TO*>(P.aux);
+  const float bias = !add_bias ? 0.f
+                     : P.in_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(P.bias)[n])
+                                 : __half2float(reinterpret_cast<const __half*>(P.bias)[n]);
+  for (int r0 = 0; r0 < rows; r0 += 8) {
+    float v[8], x[8], old[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = from_f<TO>(v[e]);
-      }
-      *reinterpret_cast<uint4*>(p) = *reinterpret_cast<uint4*>(o);
-    } else {
-      float4* q = reinterpret_cast<float4*>(p);
-      if (accumulate == 2) {
-        atomicAdd(q, make_float4(v[0], v[1], v[2], v[3]));
-        atomicAdd(q + 1, make_float4(v[4], v[5], v[6], v[7]));
-      } else {
-        float4 a = make_float4(v[0], v[1], v[2], v[3]), b = make_float4(v[4], v[5], v[6], v[7]);
-        if (accumulate) {
-          float4 c0 = q[0], c1 = q[1];
-          a.x += c0.x; a.y += c0.y; a.z += c0.z; a.w += c0.w;
-          b.x += c1.x; b.y += c1.y; b.z += c1.z; b.w += c1.w;
-        }
-        q[0] = a;
-        q[1] = b;
-      }
+    for (int u = 0; u < 8; ++u) {
+      const int64_t off = (m0 + min(r0 + u, rows - 1)) * P.ldc + n;
+      v[u] = P.alpha * stage[(r0 + u) * 32 + (lane ^ (r0 + u))] + bias;
+      x[u] = P.aux_mode ? to_f(aux[off]) : 0.f;
+      old[u] = P.accumulate == 1 || (P.accumulate && sizeof(TO) == 2) ? to_f(C[off]) : 0.f;
     }
-  } else {
-    for (int e = 0; e < n_valid; ++e) {
-      if (accumulate == 2 && sizeof(TO) == 4) atomicAdd(reinterpret_cast<float*>(p) + e, v[e]);
-      else p[e] = from_f<TO>(accumulate ? to_f(p[e]) + v[e] : v[e]);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (r0 + u >= rows) break;
+      const int64_t off = (m0 + r0 + u) * P.ldc + n;
+      if (pre) pre[off] = from_f<TO>((P.act & kActStoreGrad) ? act_grad(v[u], P.act) : v[u]);
+      float y = act_apply_tc(v[u], P.act & 0xff);
+      if (P.aux_mode) y = aux_apply(y, x[u], P.aux_mode);
+      if (P.accumulate == 2 && sizeof(TO) == 4) atomicAdd(reinterpret_cast<float*>(C) + off, y);
+      else C[off] = from_f<TO>(y + old[u]);
     }
   }
 }
@@ -590,7 +591,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       // warp-uniform outcome: tcgen05.ld below needs all 32 lanes together
       if (!__all_sync(0xffffffffu, mbar_wait(accf_bar(buf), acc_phase, abort_flag))) { ok = false; break; }
       tc_fence_after();
-      const int64_t row = m0 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
       if (P.tma_store) {
         uint8_t* stage = epi_stage + (warp - 2) * 4096;
@@ -602,53 +602,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           else fine = epilogue_staged<BN, float>(P, &tmC, &tmPre, &tmAux, taddr, stage, lane, y0, n0, add_bias, sidx, col_begin, my_aux_bar, aux_phase, aux_pre, abort_flag, stage2, my_aux_bar2, &aux_phase2, aux_pre2);
           if (!fine) { ok = false; break; }
         }
-      } else
+      } else {
+        float* const stage = reinterpret_cast<float*>(epi_stage + (warp - 2) * 4096);
+        const int rows = (int)(P.M - m0 - quarter * 32 < 32 ? P.M - m0 - quarter * 32 : 32);
 #pragma unroll 1
-      for (int c = col_begin / 32; c < (col_begin + BN / 2) / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c * 32, r);
-        tmem_ld_wait();
-        const int64_t col0 = n0 + c * 32;
-        if (row < P.M && col0 < P.N) {
-#pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int64_t col = col0 + g8 * 8;
-            if (col >= P.N) break;
-            const int n_valid = (int)(P.N - col < 8 ? P.N - col : 8);
-            float v[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              float x = P.alpha * __uint_as_float(r[g8 * 8 + e]);
-              if (add_bias && e < n_valid)
-                x += P.in_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(P.bias)[col + e])
-                               : __half2float(reinterpret_cast<const __half*>(P.bias)[col + e]);
-              v[e] = x;
-            }
-            const int64_t off = row * P.ldc + col;
-            if (P.preact) {
-              float pv[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) pv[e] = (P.act & kActStoreGrad) ? act_grad(v[e], P.act) : v[e];
-              if (P.out_dtype == MT_F16) store8(reinterpret_cast<__half*>(P.preact) + off, pv, n_valid, P.vec_store, 0);
-              else if (P.out_dtype == MT_BF16) store8(reinterpret_cast<__nv_bfloat16*>(P.preact) + off, pv, n_valid, P.vec_store, 0);
-              else store8(reinterpret_cast<float*>(P.preact) + off, pv, n_valid, P.vec_store, 0);
-            }
-            if ((P.act & 0xff) != MT_ACT_NONE) {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[e] = act_apply_tc(v[e], P.act & 0xff);
-            }
-            if (P.aux_mode) {
-              for (int e = 0; e < n_valid; ++e) {
-                const float a = P.out_dtype == MT_F16 ? __half2float(reinterpret_cast<const __half*>(P.aux)[off + e])
-                              : P.out_dtype == MT_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(P.aux)[off + e])
-                                                       : reinterpret_cast<const float*>(P.aux)[off + e];
-                v[e] = aux_apply(v[e], a, P.aux_mode);
-              }
-            }
-            if (P.out_dtype == MT_F16) store8(reinterpret_cast<__half*>(P.C) + off, v, n_valid, P.vec_store, P.accumulate);
-            else if (P.out_dtype == MT_BF16) store8(reinterpret_cast<__nv_bfloat16*>(P.C) + off, v, n_valid, P.vec_store, P.accumulate);
-            else store8(reinterpret_cast<float*>(P.C) + off, v, n_valid, P.vec_store, P.accumulate);
-          }
+        for (int c = col_begin / 32; c < (col_begin + BN / 2) / 32; ++c) {
+          if (n0 + c * 32 >= P.N || rows <= 0) break;    // warp-uniform
+          uint32_t r[32];
+          tmem_ld32(taddr + c * 32, r);
+          tmem_ld_wait();
+          if (P.out_dtype == MT_F16) epilogue_rows<__half>(P, r, stage, lane, m0 + quarter * 32, rows, n0 + c * 32 + lane, add_bias);
+          else if (P.out_dtype == MT_BF16) epilogue_rows<__nv_bfloat16>(P, r, stage, lane, m0 + quarter * 32, rows, n0 + c * 32 + lane, add_bias);
+          else epilogue_rows<float>(P, r, stage, lane, m0 + quarter * 32, rows, n0 + c * 32 + lane, add_bias);
         }
       }
       tc_fence_before();
@@ -818,7 +783,7 @@ static int launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CU
 
 // Number of two-CTA clusters of the pair kernel that are resident at once on
 // this device (an SM without a free partner in its GPC hosts none).
-static int resident_pairs() {
+int resident_cta_pairs() {
   static std::atomic<int> cached[16];      // per device; racing first calls compute the same number
   int dev = 0;
   cudaGetDevice(&dev);
@@ -862,7 +827,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t st) {
   int best_bn = 256, best_splits = 1;
   bool best_pair = false;
   double best = -1.0;
-  const int pairs_avail = resident_pairs();
+  const int pairs_avail = resident_cta_pairs();
   for (int pair = 0; pair < 2; ++pair) {
     if (pair && (g_tile_policy == 1 || g.M <= BM)) continue;
     if (!pair && g_tile_policy == 2 && g.M > BM) continue;
@@ -898,8 +863,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t st) {
   P.M = g.M; P.N = g.N; P.K = g.K; P.ldc = g.ldc;
   P.out_dtype = g.out_dtype; P.in_bf16 = g.in_dtype == MT_BF16; P.act = g.act; P.accumulate = g.accumulate;
   P.alpha = g.alpha;
-  const int out_vec = g.out_dtype == MT_F32 ? 4 : 8;
-  P.vec_store = aligned16(g.C) && (!g.preact || aligned16(g.preact)) && g.ldc % out_vec == 0;
   P.tiles_m = pair ? (int)((g.M + 2 * BM - 1) / (2 * BM)) : tiles_m;
   P.tiles_n = (int)((g.N + bn - 1) / bn);
   P.splits = best_splits;
