@@ -1,6 +1,6 @@
-// CUDA-core GEMM with fp32 accumulation: the full-precision path for fp32
-// operands (tensor cores would round to tf32) and the fallback for half
-// operands whose pointers or strides TMA cannot address. 64x64x16 tiles,
+// CUDA-core GEMM with fp32 accumulation: small products in fp32 or with pointers
+// or pitches that TMA cannot address (gemm_split.cu takes the larger ones), and
+// the independent check of the tensor-core kernels. 64x64x16 tiles,
 // 256 threads, 4x4 outputs per thread, any strides / transposes / tails.
 #include "common.cuh"
 #include "gemm.cuh"

@@ -11,12 +11,14 @@
 // Relative error against 64 bits (2-norm, normal data): K = 256 8.6e-8 (FMA chain 2.9e-7), 768 1.0e-7 (5.0e-7),
 // 4096 1.1e-7 (1.1e-6), 8192 2.2e-7 (1.6e-6).
 //
-// One 128 x 128 tile per CTA (persistent): a slot of the ring holds one plane of A and of B (2 x 16 KB); the
-// 24 MMAs of a 64-deep slice (1536 tensor cycles) read 96 KB, 64 B per clock and SM. Where tiles are few
+// Persistent. A slot of a CTA's ring holds 128 rows of one plane of A and of B (2 x 16 KB), a 64-deep slice of fp32
+// operands three slots. A CTA pair (cta_group::2) works on a 256 x 256 tile: the 24 MMAs of a slice last 3072 tensor
+// cycles while the ring's other half fills. A single CTA's 128 x 128 tile lasts 1536 and waits for its 96 KB (64 B per clock
+// and SM, and as long a way from L2 as the MMAs take); it is there for products with too few tiles. Where even those are few
 // (weight gradients of small layers), K is split over a cluster of up to eight CTAs whose sums meet
 // through distributed shared memory in a fixed order: no atomics, the same bits every time.
-// fp32: 8192 x 768 -> 3072 1414 -> 369 us, its weight gradient 1529 -> 258, 4096 x 256 -> 1024 102 -> 47, 256 x 4096 x 256
-// 209 -> 25; bf16 with odd pitches: 3885 x 50257 -> 768 15158 -> 719 us, 50257 x 3885 -> 768 12345 -> 658.
+// fp32: 8192 x 768 -> 3072 1414 -> 202 us, its weight gradient 1529 -> 260, 4096 x 256 -> 1024 102 -> 25, 256 x 4096 x 256
+// 209 -> 25; bf16 with odd pitches and fp32 output: 50257 x 3885 -> 768 12345 -> 526 us.
 //
 // A result that is not finite (an operand is, or |x| > 3.39e38 rounds to bf16 infinity) is computed
 // again as a plain fp32 dot product, so infinities and NaNs come out as fp32 arithmetic gives them.
@@ -89,10 +91,12 @@ __device__ __forceinline__ void split_finish(const SplitParams& P, float v, floa
   store_typed(P.C, off, P.out_dtype, v);
 }
 
-template <bool F32, bool A_MN, bool B_MN>
+template <bool F32, bool A_MN, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(kSpThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitParams P) {
   constexpr int PLANES = F32 ? 3 : 1;
+  constexpr int TM = PAIR ? 256 : 128, TN = PAIR ? 256 : 128;      // tile of a CTA or a pair; either way a CTA stages 128 rows of A and of B
+  constexpr int NC = TN / 2;                         // columns an epilogue warp holds
   extern __shared__ uint8_t sp_smem[];
   const uint32_t raw = smem_u32(sp_smem);
   const uint32_t base = (raw + 1023u) & ~1023u;      // the 128-byte swizzle repeats every 1024 bytes
@@ -107,19 +111,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bar_ptr + 8 * (2 * kSpSlots + 4));
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int csize = P.csize;
+  const int csize = PAIR ? 1 : P.csize;              // CTAs that split K
+  const int prank = PAIR ? (int)cluster_ctarank() : 0;
   const int rank = csize > 1 ? (int)cluster_ctarank() : 0;
-  const int worker = (int)blockIdx.x / csize, workers = (int)gridDim.x / csize;
+  const int per_worker = PAIR ? 2 : csize;
+  const int worker = (int)blockIdx.x / per_worker, workers = (int)gridDim.x / per_worker;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSpSlots; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), kSpEpiWarps); }
+    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), PAIR ? 2 * kSpEpiWarps : kSpEpiWarps); }
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 2 * kSpN); tmem_relinquish(); }
+  if (warp == 1) {
+    if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), 2 * TN); tmem_relinquish_pair(); }
+    else { tmem_alloc(smem_u32(tmem_slot), 2 * TN); tmem_relinquish(); }
+  }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();                      // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   griddep_launch();
@@ -137,22 +147,27 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       long long issued = 0;
       bool ok = true;
       for (int t = worker; t < total && ok; t += workers) {
-        const int m0 = (P.n_fast ? t / P.tiles_n : t % P.tiles_m) * kSpM, n0 = (P.n_fast ? t % P.tiles_n : t / P.tiles_m) * kSpN;
+        const int m0 = (P.n_fast ? t / P.tiles_n : t % P.tiles_m) * TM + prank * 128, n0 = (P.n_fast ? t % P.tiles_n : t / P.tiles_m) * TN + prank * 128;
         for (int kb = kb0; kb < kb1 && ok; ++kb) {
           for (int pl = 0; pl < PLANES; ++pl) {
             if (!mbar_wait(empty_bar(slot), phase ^ 1u, abort_flag)) { ok = false; break; }
-            const uint32_t sa = base + slot * kSpSlot, sb = sa + kSpPlane, bar = full_bar(slot);
-            mbar_expect_tx(bar, kSpSlot);
-            if (!A_MN) tma_load_3d(sa, &tmA, bar, kb * kSpK, m0, pl);
-            else for (int j = 0; j < 2; ++j) tma_load_3d(sa + j * (kSpK * 128), &tmA, bar, m0 + j * 64, kb * kSpK, pl);
-            if (!B_MN) tma_load_3d(sb, &tmB, bar, kb * kSpK, n0, pl);
-            else for (int j = 0; j < 2; ++j) tma_load_3d(sb + j * (kSpK * 128), &tmB, bar, n0 + j * 64, kb * kSpK, pl);
+            const uint32_t sa = base + slot * kSpSlot, sb = sa + kSpPlane;
+            const uint32_t bar = PAIR ? mapa_shared(full_bar(slot), 0) : full_bar(slot);     // rank 0 counts both CTAs' copies
+            if (prank == 0) mbar_expect_tx(full_bar(slot), PAIR ? 2 * kSpSlot : kSpSlot);
+            auto load = [&](uint32_t dst, const CUtensorMap* map, int x, int y) {
+              if (PAIR) tma_load_3d_pair(dst, map, bar, x, y, pl);
+              else tma_load_3d(dst, map, bar, x, y, pl);
+            };
+            if (!A_MN) load(sa, &tmA, kb * kSpK, m0);
+            else for (int j = 0; j < 2; ++j) load(sa + j * (kSpK * 128), &tmA, m0 + j * 64, kb * kSpK);
+            if (!B_MN) load(sb, &tmB, kb * kSpK, n0);
+            else for (int j = 0; j < 2; ++j) load(sb + j * (kSpK * 128), &tmB, n0 + j * 64, kb * kSpK);
             ++issued;
             if (++slot == kSpSlots) { slot = 0; phase ^= 1u; }
           }
         }
       }
-      if (!ok) {                                       // bounded: the copies in flight land before shared memory goes away
+      if (!ok && prank == 0) {                         // bounded: the copies in flight land before shared memory goes away
         const long long n = issued < kSpSlots ? issued : kSpSlots;
         int s = slot;
         uint32_t ph = phase;
@@ -165,8 +180,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer --
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16(F32 || P.in_dtype == MT_BF16, A_MN, B_MN, kSpM, kSpN);
+    if (lane == 0 && prank == 0) {
+      const uint32_t idesc = idesc_f16(F32 || P.in_dtype == MT_BF16, A_MN, B_MN, TM, TN);
+      auto commit = [&](uint32_t bar) { if (PAIR) umma_commit_pair(bar); else umma_commit(bar); };
       int slot = 0, it = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -175,7 +191,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const int buf = it & 1;
           if (!mbar_wait(acce_bar(buf), ((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t d = tmem_base + buf * kSpN;
+          const uint32_t d = tmem_base + buf * TN;
           const int ke = min(kb1, kc + P.chunk);
           for (int kb = kc; kb < ke && ok; ++kb) {
             // the slots of a slice are neighbours: kSpSlots is a multiple of PLANES
@@ -190,7 +206,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 a[k] = A_MN ? smem_desc_sw128(sa + k * 2048, kSpK * 128, 1024) : smem_desc_sw128(sa + k * 32, 16, 1024);
                 b[k] = B_MN ? smem_desc_sw128(sb + k * 2048, kSpK * 128, 1024) : smem_desc_sw128(sb + k * 32, 16, 1024);
               }
-              umma_f16_x4(d, a, b, idesc, acc);
+              if (PAIR) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_f16_pair(d, a[k], b[k], idesc, k ? 1u : acc);
+              } else {
+                umma_f16_x4(d, a, b, idesc, acc);
+              }
             };
             const uint32_t acc = kb > kc ? 1u : 0u;
             if (F32) {
@@ -203,51 +224,56 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             } else {
               product(0, 0, acc);
             }
-            for (int pl = 0; pl < PLANES; ++pl) umma_commit(empty_bar(slot + pl));
+            for (int pl = 0; pl < PLANES; ++pl) commit(empty_bar(slot + pl));
             slot += PLANES;
             if (slot == kSpSlots) { slot = 0; phase ^= 1u; }
           }
-          if (ok) umma_commit(accf_bar(buf));
+          if (ok) commit(accf_bar(buf));
         }
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue --
-    const int quarter = warp & 3, c0 = ((warp - 2) >> 2) * (kSpN / 2);      // 32 rows, 64 columns of the tile
+    const int quarter = warp & 3, c0 = ((warp - 2) >> 2) * NC;      // 32 rows, half of the tile's columns
     float* const stage = stages + (warp - 2) * (32 * 33);
     int it = 0;
     bool ok = true;
     for (int t = worker; t < total && ok; t += workers) {
-      const int64_t m0 = (int64_t)(P.n_fast ? t / P.tiles_n : t % P.tiles_m) * kSpM + quarter * 32;
-      const int64_t n0 = (int64_t)(P.n_fast ? t % P.tiles_n : t / P.tiles_m) * kSpN + c0;
-      float acc[64];
+      const int64_t m0 = (int64_t)(P.n_fast ? t / P.tiles_n : t % P.tiles_m) * TM + prank * 128 + quarter * 32;
+      const int64_t n0 = (int64_t)(P.n_fast ? t % P.tiles_n : t / P.tiles_m) * TN + c0;
+      float acc[NC];
 #pragma unroll
-      for (int e = 0; e < 64; ++e) acc[e] = 0.f;
+      for (int e = 0; e < NC; ++e) acc[e] = 0.f;
       for (int kc = kb0; kc < kb1; kc += P.chunk, ++it) {
         const int buf = it & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(accf_bar(buf), (it >> 1) & 1, abort_flag))) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * kSpN + c0;
-        uint32_t r[64];
-        tmem_ld32(taddr, r);
-        tmem_ld32(taddr + 32, r + 32);
-        tmem_ld_wait();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TN + c0;
+#pragma unroll
+        for (int h = 0; h < NC; h += 32) {
+          uint32_t r[32];
+          tmem_ld32(taddr + h, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) acc[h + e] += __uint_as_float(r[e]);
+        }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(acce_bar(buf));
-#pragma unroll
-        for (int e = 0; e < 64; ++e) acc[e] += __uint_as_float(r[e]);
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster(mapa_shared(acce_bar(buf), 0));
+          else mbar_arrive(acce_bar(buf));
+        }
       }
       if (!ok) break;
       if (csize > 1) {
         // all copies and MMAs of this CTA are done: its ring holds the sums for the cluster
         float* rows = reinterpret_cast<float*>(base_ptr) + (quarter * 32 + lane) * kSpPitch + c0;
 #pragma unroll
-        for (int e = 0; e < 64; ++e) rows[e] = acc[e];
+        for (int e = 0; e < NC; ++e) rows[e] = acc[e];
       } else {
         // thread = row becomes lane = column: rows of 128 bytes to and from global memory, any pitch
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < NC / 32; ++h) {
           const int64_t n = n0 + h * 32 + lane;
           __syncwarp();
 #pragma unroll
@@ -256,18 +282,28 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (n < P.N) {
             const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
             const int rows = (int)min((int64_t)32, P.M - m0);
-            for (int r0 = 0; r0 < rows; r0 += 8) {            // eight rows' reads in flight at a time
-              float v[8], aux[8], old[8];
+            const bool plain = !P.preact && !P.act && !P.aux_mode && !P.accumulate && P.out_dtype == MT_F32;
+            float* const c = (float*)P.C + m0 * P.ldc + n;
+            for (int r0 = 0; r0 < rows; r0 += 8) {
+              float v[8];
+              bool fine = plain && r0 + 8 <= rows;
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
-                const int64_t off = (m0 + min(r0 + u, rows - 1)) * P.ldc + n;
                 v[u] = stage[(r0 + u) * 33 + lane];
-                aux[u] = P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f;
-                old[u] = P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f;
+                fine = fine && (!F32 || fabsf(v[u]) <= 3.402823466e38f);
               }
+              if (fine) {
 #pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (r0 + u < rows) split_finish<F32>(P, v[u], bias, aux[u], old[u], m0 + r0 + u, n);
+                for (int u = 0; u < 8; ++u) c[(r0 + u) * P.ldc] = P.alpha * v[u] + bias;
+              } else {
+                // (kept small: eight copies of it in a row ran 15 % slower, on instruction fetches)
+#pragma unroll 2
+                for (int r = r0; r < min(r0 + 8, rows); ++r) {
+                  const int64_t off = (m0 + r) * P.ldc + n;
+                  split_finish<F32>(P, stage[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
+                                    P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
+                }
+              }
             }
           }
         }
@@ -278,7 +314,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   // ------------------------------------------------- sums of a cluster, teardown --
   tc_fence_before();
   __syncthreads();
-  if (csize > 1) {
+  if (PAIR) cluster_sync_all();                        // neither CTA leaves, nor frees tensor memory, while its peer still works
+  if (!PAIR && csize > 1) {
     cluster_sync_all();
     if (worker < total) {
       const int64_t m0 = (int64_t)(P.n_fast ? worker / P.tiles_n : worker % P.tiles_m) * kSpM;
@@ -320,7 +357,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (threadIdx.x == 0 && *abort_flag && P.flag) atomicMax(P.flag, 106);   // a bounded wait expired
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * kSpN);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 2 * TN);
+    else tmem_dealloc(tmem_base, 2 * TN);
   }
 }
 
@@ -379,7 +417,7 @@ prepare_kernel(const PrepareJob a, const PrepareJob b) {
 // The CUDA-core kernel takes about 8 us and 0.05 us per k for each 64 x 64 tile an SM has (measured in fp32: 256^3
 // 21 us, 4096 x 256 x 256 29, 4096 x 256 x 65 15, 4096 x 1024 x 256 102); this path 15-23 us for small products, most of
 // it the host's two launches, allocation and tensor maps (256^3 17 us, 4096 x 256 x 256 20, 4096 x 256 x 65 23).
-constexpr double kSplitMinUs = 24.0;
+constexpr double kSplitMinUs = 30.0;
 
 bool gemm_split_supported(const GemmArgs& g) {
   if (g.M < 16 || g.N < 16 || g.K < 16) return false;
@@ -388,9 +426,9 @@ bool gemm_split_supported(const GemmArgs& g) {
   return 8.0 + 0.05 * (double)g.K * (tiles > 1.0 ? tiles : 1.0) >= kSplitMinUs;
 }
 
-template <bool F32, bool A_MN, bool B_MN>
+template <bool F32, bool A_MN, bool B_MN, bool PAIR>
 static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const SplitParams& P, int grid, cudaStream_t st) {
-  auto kern = gemm_split_kernel<F32, A_MN, B_MN>;
+  auto kern = gemm_split_kernel<F32, A_MN, B_MN, PAIR>;
   static std::atomic<bool> ready[16];      // per device; racing first calls set the same attribute twice, harmlessly
   int dev = 0;
   cudaGetDevice(&dev);
@@ -405,7 +443,7 @@ static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const Spli
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)P.csize;
+  attr[0].val.clusterDim.x = PAIR ? 2u : (unsigned)P.csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -475,15 +513,14 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
   P.M = g.M; P.N = g.N; P.K = g.K; P.lda = g.lda; P.ldb = g.ldb; P.ldc = g.ldc;
   P.trans_a = g.trans_a; P.trans_b = g.trans_b; P.in_dtype = g.in_dtype; P.out_dtype = g.out_dtype;
   P.act = g.act; P.aux_mode = g.aux_mode; P.accumulate = g.accumulate; P.alpha = g.alpha;
-  P.tiles_m = (int)((g.M + kSpM - 1) / kSpM);
-  P.tiles_n = (int)((g.N + kSpN - 1) / kSpN);
   P.kb_total = (int)((g.K + kSpK - 1) / kSpK);
   P.chunk = f32 || g.out_dtype == MT_F32 ? 1 : 4;      // a half output's own rounding hides what four slices lose
   P.flag = device_flag_ptr();
   // Neighbouring tiles share the larger operand's panel unless it fits the L2 anyway.
   P.n_fast = g.M > g.N ? 1 : 0;
-  const int sms = sm_count();
-  const long long tiles = (long long)P.tiles_m * P.tiles_n;
+  const int sms = sm_count(), pairs = resident_cta_pairs();
+  auto tiles_of = [&](int t) { return ((g.M + t - 1) / t) * ((g.N + t - 1) / t); };
+  long long tiles = tiles_of(128);
   // K over a cluster while that leaves no CTA waiting for an SM and each at least two slices.
   P.csize = 1;
   while (P.csize < 8 && tiles * P.csize * 2 <= sms && P.kb_total >= 4 * P.csize) P.csize *= 2;
@@ -492,14 +529,30 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
     P.csize /= 2;
     P.kb_per_rank = (P.kb_total + P.csize - 1) / P.csize;
   }
-  const int grid = P.csize > 1 ? (int)tiles * P.csize : (int)(tiles < sms ? tiles : sms);
+  // A pair's 256 x 256 tile needs half the operand bytes per multiplication: a slice takes it about 4300
+  // cycles, a single CTA's 128 x 128 tile 3600 (one plane: 1990, 1770); which one is ahead is a matter of how many rounds
+  // of tiles each leaves on the chip (fp32 8192 x 768 -> 3072: pair 202 us, single 423; 3072 x 8192 x 768: 308, 260).
+  const double kb_one = f32 ? 3600.0 : 1770.0, kb_pair = f32 ? 4300.0 : 1990.0;
+  const double one = (double)((tiles * P.csize + sms - 1) / sms) * (P.kb_per_rank * kb_one + 4000.0);
+  const double two = (double)((tiles_of(256) + pairs - 1) / pairs) * (P.kb_total * kb_pair + 6000.0);
+  const bool pair = two < one;
+  if (pair) {
+    tiles = tiles_of(256);
+    P.csize = 1;
+    P.kb_per_rank = P.kb_total;
+  }
+  const int64_t t = pair ? 256 : 128;
+  P.tiles_m = (int)((g.M + t - 1) / t);
+  P.tiles_n = (int)((g.N + t - 1) / t);
+  const int grid = pair ? 2 * (int)(tiles < pairs ? tiles : pairs) : P.csize > 1 ? (int)tiles * P.csize : (int)(tiles < sms ? tiles : sms);
+#define MT_SPLIT_ORDER(F, A, B) \
+  (pair ? launch_split<F, A, B, true>(map[0], map[1], P, grid, st) : launch_split<F, A, B, false>(map[0], map[1], P, grid, st))
 #define MT_SPLIT(F)                                                                       \
-  (mn[0] ? (mn[1] ? launch_split<F, true, true>(map[0], map[1], P, grid, st)              \
-                  : launch_split<F, true, false>(map[0], map[1], P, grid, st))            \
-         : (mn[1] ? launch_split<F, false, true>(map[0], map[1], P, grid, st)             \
-                  : launch_split<F, false, false>(map[0], map[1], P, grid, st)))
+  (mn[0] ? (mn[1] ? MT_SPLIT_ORDER(F, true, true) : MT_SPLIT_ORDER(F, true, false))       \
+         : (mn[1] ? MT_SPLIT_ORDER(F, false, true) : MT_SPLIT_ORDER(F, false, false)))
   return f32 ? MT_SPLIT(true) : MT_SPLIT(false);
 #undef MT_SPLIT
+#undef MT_SPLIT_ORDER
 }
 
 }  // namespace mt

@@ -28,11 +28,11 @@ def bound(K):
     return (24 * 2 + K / 64 + 2) * 2.0 ** -24
 
 
-# one tile and less, ragged in every direction, pitches of 4, 8, 12 and odd bytes; few tiles with K split over 2, 4 and
+# (each large enough for this path) one tile and less, ragged in every direction, pitches of 4, 8, 12 and odd bytes; few tiles with K split over 2, 4 and
 # 8 CTAs (512, 1000, 4096); more tiles than SMs
 @pytest.mark.parametrize("ta,tb", ORDERS)
-@pytest.mark.parametrize("M,N,K", [(128, 128, 512), (129, 65, 1001), (72, 2000, 384), (67, 131, 1000), (256, 264, 4096), (300, 77, 4099),
-                                   (1700, 1666, 70)])
+@pytest.mark.parametrize("M,N,K", [(128, 128, 512), (129, 65, 1001), (72, 2000, 512), (67, 131, 1000), (256, 264, 4096), (300, 77, 4099),
+                                   (1700, 1666, 90), (1630, 1560, 100)])
 def test_fp32_products(mt, ta, tb, M, N, K):
     r = np.random.default_rng(M + N + K)
     a = r.standard_normal((K, M) if ta else (M, K)).astype(np.float32)
@@ -45,7 +45,7 @@ def test_fp32_products(mt, ta, tb, M, N, K):
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("ta,tb", ORDERS)
-@pytest.mark.parametrize("M,N,K", [(129, 65, 1001), (300, 77, 4099), (1700, 1665, 71), (128, 264, 401)])
+@pytest.mark.parametrize("M,N,K", [(129, 65, 1001), (300, 77, 4099), (1700, 1665, 91), (128, 264, 501)])
 def test_half_products_with_odd_pitches(mt, dtype, ta, tb, M, N, K):
     r = np.random.default_rng(M + N + K)
     a, b = rnd(r.standard_normal((K, M) if ta else (M, K)), dtype), rnd(r.standard_normal((N, K) if tb else (K, N)), dtype)
@@ -58,7 +58,7 @@ def test_half_products_with_odd_pitches(mt, dtype, ta, tb, M, N, K):
     no_device_flag(mt)
 
 
-@pytest.mark.parametrize("M,N,K", [(300, 260, 400), (130, 70, 2000)])          # one CTA per tile, a cluster per tile
+@pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000)])          # one CTA per tile, a cluster per tile
 def test_epilogues_match_the_cuda_core_kernel(mt, M, N, K):
     F = mt.fused_ops
     r = np.random.default_rng(5)
@@ -87,7 +87,7 @@ def test_epilogues_match_the_cuda_core_kernel(mt, M, N, K):
     no_device_flag(mt)
 
 
-@pytest.mark.parametrize("M,N,K", [(300, 260, 400), (130, 70, 2000)])
+@pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000)])
 def test_values_that_are_not_finite_come_out_as_in_fp32(mt, M, N, K):
     r = np.random.default_rng(6)
     a, b = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
