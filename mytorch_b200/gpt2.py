@@ -192,27 +192,36 @@ def _init_weights(module):     # gpt2_trainer/gpt2.py:376-389
 
 
 def _plan(model):
-    """Describes the model to the library's whole-model forward (see infer.Plan)."""
+    """What the library's whole-model forward needs to know of the model as it is now (see
+    infer.plan_of); None when it does not cover it."""
     cfg, plain = model.config, infer.plain
-    ok = plain(model, GPT2) and plain(model.embeddings, Embeddings) and plain(model.final_layer_norm, nn.LayerNorm) \
-        and plain(model.lm_head, nn.Linear) and model.lm_head.act_func is None
-    rows = []
+    e, lnf, head = model.embeddings, model.final_layer_norm, model.lm_head
+    if not (infer.unpatched(_METHODS) and plain(model, GPT2) and plain(e, Embeddings) and plain(lnf, nn.LayerNorm)
+            and plain(head, nn.Linear) and head.act_func is None):
+        return None
+    H, E = cfg.num_heads, cfg.embed_dim
+    eps = {lnf.eps}
+    found = infer.arrays(e.char_embeddings.weight, e.position_embeddings.weight, lnf.weight, lnf.bias, head.weight, head.bias) + [None, None]
     for b in model.blocks:
-        ok = ok and plain(b, TransformerBlock) and plain(b.attention, Attention) and plain(b.feedforward, FeedForward)
-        if not ok:
-            break
-        a, f = b.attention, b.feedforward
-        linears = (a.qkv_proj, a.out_proj, f.intermediate_dense, f.out_proj)
-        ok = all(plain(m, nn.Linear) for m in linears) and plain(b.layernorm1, nn.LayerNorm) and plain(b.layernorm2, nn.LayerNorm) \
-            and a.proj_drop.p == f.intermediate_dropout.p == f.output_dropout.p == 0.0 \
-            and [m.act_func for m in linears] == [None, None, "gelu", None] and a.num_heads == cfg.num_heads
-        rows.append((b.layernorm1, b.layernorm2, a.qkv_proj, None, None, a.out_proj, f.intermediate_dense, f.out_proj))
-    if not ok:
-        return infer.NoPlan(model.blocks)
-    e = model.embeddings
-    return infer.Plan(model, 0, {"wte": e.char_embeddings, "wpe": e.position_embeddings, "lnf": model.final_layer_norm,
-                                 "head": model.lm_head}, model.blocks, rows, cfg.num_heads, cfg.num_heads,
-                      cfg.embed_dim * cfg.mlp_ratio, cfg.vocab_size)
+        if not plain(b, TransformerBlock):
+            return None
+        a, f, n1, n2 = b.attention, b.feedforward, b.layernorm1, b.layernorm2
+        if not (plain(a, Attention) and "_cached_attention" not in a.__dict__ and plain(f, FeedForward) and plain(n1, nn.LayerNorm)
+                and plain(n2, nn.LayerNorm) and a.num_heads == H and a.embed_dim == E and a.head_dim * H == E):
+            return None
+        qkv, out, up, down = a.qkv_proj, a.out_proj, f.intermediate_dense, f.out_proj
+        if not (plain(qkv, nn.Linear) and plain(out, nn.Linear) and plain(up, nn.Linear) and plain(down, nn.Linear)
+                and qkv.act_func is None and out.act_func is None and up.act_func == "gelu" and down.act_func is None):
+            return None
+        for drop in (a.proj_drop, f.intermediate_dropout, f.output_dropout):
+            if not (plain(drop, nn.Dropout) and drop.p == 0.0):
+                return None
+        eps.update((n1.eps, n2.eps))
+        found += infer.arrays(n1.weight, n1.bias, n2.weight, n2.bias, qkv.weight, None, None, out.weight, up.weight, down.weight,
+                              qkv.bias, None, None, out.bias, up.bias, down.bias)
+    if len(eps) > 1:
+        return None
+    return (0, len(model.blocks), E, E * cfg.mlp_ratio, H, H, cfg.vocab_size, eps.pop()), found
 
 
 class GPT2(nn.Module):
@@ -236,16 +245,16 @@ class GPT2(nn.Module):
         self._gradient_checkpointing_enabled = True
 
     def _planned(self, plan, ids, cache=None, last_only=False):
-        """The whole forward as one library call (no graph); None when the cache's layers differ."""
+        """The whole forward as one library call (no graph); None when the cache is not as this model
+        would have made it."""
         B, T = ids.shape
+        past = cache.get_seq_len() if cache is not None else 0
+        assert past + T <= (min(plan.positions, self.config.max_seq_len) if past else plan.positions), "position table exhausted"
         if cache is None:
-            assert T <= self.config.max_seq_len, "position table exhausted"
             return plan.run(ids, last_only=last_only)
         cfg, n = self.config, cache.max_seq_len
         D = plan.head_dim
-        past = cache.get_seq_len()
-        assert past + T <= cfg.max_seq_len, "position table exhausted"
-        if not cache.reserve(B, cfg.num_heads, D, plan.dtype) or T > n or (past and D not in (64, 128)):
+        if T > n or (past and D not in (64, 128)) or not cache.reserve(B, cfg.num_heads, D, plan.dtype):
             return None
         L = len(cache.key_cache)
         ptrs = C.c_void_p * L
@@ -277,17 +286,14 @@ class GPT2(nn.Module):
         logits = self.lm_head(x)
         return logits if cache is None else (logits, cache)
 
-    def _generate_greedy(self, plan, ids, cache, n):
-        """The arg-max stays on the device and is the next step's input: the host queues all steps
-        and reads the ids back once."""
-        out = DeviceArray.empty((ids.shape[0], n), "int32")
-        feed = Tensor(ids).data
-        for i in range(n):
-            logits = self._planned(plan, feed, cache, last_only=True)
-            if logits is None:
-                return None
-            feed = infer.greedy(logits, out, i)
-        return out.numpy()
+    def _next_logits(self, feed, cache):
+        """Logits [B, 1 or T, V] after the ids `feed`; the last position is the next token's."""
+        plan = infer.plan_of(self, _plan)
+        out = self._planned(plan, feed, cache, last_only=True) if plan is not None and feed.size else None
+        if out is None:
+            out = self.forward(Tensor(feed), cache=cache)
+            out = (out if cache is None else out[0]).data
+        return out
 
     def generate(self, input_ids, max_new_tokens, temperature=1.0, top_k=None, use_cache=True, seed=None):
         """Autoregressive sampling as in gpt2_trainer/inference_gpt2.py:137-174: the prompt fills
@@ -299,16 +305,10 @@ class GPT2(nn.Module):
         cache = Cache(self.config) if use_cache else None
         feed = ids
         with no_grad():
-            plan = infer.plan_of(self, _plan)
-            if plan is not None and temperature == 0 and use_cache and max_new_tokens > 0 and ids.size:
-                new = self._generate_greedy(plan, ids, cache, max_new_tokens)
-                if new is not None:
-                    return np.concatenate([ids, new], axis=1)
+            if temperature == 0 and use_cache and max_new_tokens > 0 and ids.size and infer.plan_of(self, _plan) is not None:
+                return infer.generate_greedy(self, ids, cache, max_new_tokens)
             for _ in range(max_new_tokens):
-                logits = self._planned(plan, Tensor(feed).data, cache, last_only=True) if plan is not None else None
-                if logits is None:
-                    out = self.forward(Tensor(feed), cache=cache)
-                    logits = out[0] if use_cache else out
+                logits = self._next_logits(Tensor(feed).data, cache)
                 last = logits.numpy()[:, -1, :].astype(np.float64)
                 if temperature == 0:
                     nxt = last.argmax(-1)
@@ -323,3 +323,6 @@ class GPT2(nn.Module):
                 ids = np.concatenate([ids, nxt[:, None].astype(np.int32)], axis=1)
                 feed = ids[:, -1:] if use_cache else ids[:, -self.config.max_seq_len:]
         return ids
+
+
+_METHODS = infer.methods(GPT2, Embeddings, TransformerBlock, Attention, FeedForward, nn.Linear, nn.LayerNorm, nn.Dropout)

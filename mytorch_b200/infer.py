@@ -1,88 +1,96 @@
 """Model forwards without a graph as one library call (`mt_gpt_forward`): the inference branches of
 gpt2_trainer/gpt2.py:352-374 and nanochat_trainer/core/nanochat_gpt.py:301-340.
 
-A `Plan` describes a model's weights to the library. It is kept on the model and checked on every
-use: each weight it was built from must still be the module's parameter and hold the same device
-array, so loading, casting or replacing weights makes a new plan. Models that the call does not
-cover (subclassed modules, dropout, mixed dtypes) return no plan and run op by op.
+A `Plan` describes a model's weights to the library: addresses and sizes, no reference to an array or
+a module. Every forward walks the model as it stands and compares what it finds with the kept
+description, so replaced modules, weights, tables and options take effect at once and a model's old
+arrays are not held. Models that the call does not cover (subclassed or patched modules, dropout,
+other activations, mixed dtypes, tensors of unexpected shapes) return no plan and run op by op.
 """
 import ctypes as C
 
+import numpy as np
+
 from . import _lib
-from .array import DeviceArray, stream
+from .array import DeviceArray, code, stream
 from .tensor import Tensor
 
-# norm1 w, b; norm2 w, b; q (or qkv), k, v, out, up, down weights; their biases
 _NO_STRIDES = _lib.Strides3(0, 0, 0)
+TOP, PER_BLOCK = 8, 16        # arrays of a description: the model's own, then each block's
 
 
 def plain(module, cls):
     """The module is exactly `cls` with the class's own forward."""
-    return type(module) is cls and "forward" not in module.__dict__
+    return module.__class__ is cls and "forward" not in module.__dict__
+
+
+def methods(*classes):
+    """The forwards (and Module.__call__) that the library call stands for, as they are at import."""
+    from .nn.modules import Module
+    return [(c, "forward", c.forward) for c in classes] + [(Module, "__call__", Module.__call__)]
+
+
+def unpatched(known):
+    return all(getattr(c, name) is f for c, name, f in known)
+
+
+def arrays(*tensors):
+    return [None if t is None else t.data for t in tensors]
 
 
 def greedy(logits, ids_out, column):
-    """Arg-max of every row of logits [B, 1, V] into ids_out[:, column] (int32 on the device) and as
-    the next step's ids [B, 1]."""
-    B, V = logits.shape[0], logits.shape[-1]
+    """Arg-max of every sequence's last row of logits [B, T, V] into ids_out[:, column] (int32 on the
+    device) and as the next step's ids [B, 1]."""
+    B, T, V = logits.shape
+    if T > 1:
+        logits = DeviceArray.from_numpy(logits.numpy()[:, -1:, :], logits.dtype)
     nxt = DeviceArray.empty((B, 1), "int32")
     _lib.argmax_rows(logits.ptr, nxt.ptr, ids_out.ptr + 4 * column, B, V, ids_out.shape[1], logits.code, stream())
     return nxt
 
 
+def generate_greedy(model, ids, cache, n):
+    """[ids | n tokens]: the arg-max stays on the device and is the next step's input, so the host
+    queues all steps and reads the tokens back once."""
+    out, feed = DeviceArray.empty((ids.shape[0], n), "int32"), Tensor(ids).data
+    for i in range(n):
+        feed = greedy(model._next_logits(feed, cache), out, i)
+    return np.concatenate([ids, out.numpy()], axis=1)
+
+
 class Plan:
-    def __init__(self, model, kind, modules, blocks, block_modules, heads, kv_heads, hidden, vocab, cos=None, sin=None):
-        """modules: {"wte", "wpe", "lnf", "head"} -> module or None; block_modules: per block the
-        modules in the order norm1, norm2, q, k, v, out, up, down (None = absent)."""
-        self.ok = False
-        self.blocks = list(blocks)
-        self.checks = []
-        self.keep = (cos, sin)
+    """sizes: (kind, blocks, width, hidden, heads, kv_heads, vocab, eps); found: (address, shape,
+    dtype) or None of the token and position tables, the final norm's weight and bias, the head's
+    weight and bias, the rotary tables, then per block 16 tensors in the order of `block_ptrs` in
+    mytorch_b200.h."""
 
-        def ptr(module, name):
-            t = None if module is None else getattr(module, name, None)
-            if module is not None:
-                self.checks.append((module, name, t, None if t is None else t.data))
-            return t
-
-        def address(t):
-            return None if t is None else t.data.ptr
-        top = {k: (ptr(m, "weight"), ptr(m, "bias")) for k, m in modules.items()}
-        rows = []
-        for mods in block_modules:
-            w = [ptr(m, "weight") for m in mods]
-            b = [ptr(m, "bias") for m in mods]
-            rows.append([w[0], b[0], w[1], b[1], *w[2:], *b[2:]])
-        tensors = [t for pair in top.values() for t in pair if t is not None] + [t for r in rows for t in r if t is not None]
-        dtypes = {t.dtype for t in tensors}
-        eps = {m.eps for m in [modules.get("lnf")] + [m for mods in block_modules for m in mods[:2]] if m is not None}
-        if len(dtypes) != 1 or len(eps) > 1:
+    def __init__(self, sizes, found):
+        kind, blocks, width, hidden, heads, kv_heads, vocab, eps = sizes
+        self.sizes, self.found, self.ok = sizes, found, False
+        self.blocks, self.vocab, self.head_dim = blocks, vocab, width // heads
+        D = self.head_dim
+        dtypes = {f[2] for i, f in enumerate(found) if f is not None and i not in (6, 7)}
+        table = found[6] if kind else found[1]              # rotary tables; learned positions
+        if len(dtypes) != 1 or D > 128 or table is None or found[0] is None or found[4] is None:
             return
         self.dtype = dtypes.pop()
-        flat = [address(t) for r in rows for t in r]
-        self.ptrs = (C.c_void_p * max(1, len(flat)))(*flat)
-        wte = top["wte"][0]
-        head_w, head_b = top["head"]
-        width = wte.shape[1]
-        self.c = _lib.GptModel(kind, wte.data.code, len(rows), width, hidden, heads, kv_heads, vocab, address(wte),
-                               address(top["wpe"][0]) if "wpe" in top else None, *(map(address, top["lnf"]) if "lnf" in top else (None, None)),
-                               address(head_w), address(head_b), None if cos is None else cos.ptr, None if sin is None else sin.ptr,
-                               C.cast(self.ptrs, C.c_void_p), eps.pop() if eps else 1e-5)
-        self.vocab, self.head_dim = vocab, width // heads
-        D = self.head_dim
-        q_rows = 3 * width if kind == 0 else heads * D
-        want = [(width,)] * 4 + [(q_rows, width)] + [(kv_heads * D, width)] * 2 + [(width, heads * D), (hidden, width), (width, hidden)]
-        shapes_ok = head_w.shape == (vocab, width) and all(t is None or t.shape == w for r in rows for t, w in zip(r, want))
-        self.ok = shapes_ok and D <= 128
-
-    def valid(self, blocks):
-        if len(blocks) != len(self.blocks) or any(a is not b for a, b in zip(blocks, self.blocks)):
-            return False
-        for module, name, t, data in self.checks:
-            now = getattr(module, name, None)
-            if now is not t or (t is not None and t.data is not data):
-                return False
-        return True
+        self.positions = table[1][0]
+        pos = (self.positions, D if kind else width)
+        q_rows, kv = heads * D if kind else 3 * width, kv_heads * D
+        want = [(vocab, width), pos, (width,), (width,), (vocab, width), (vocab,), pos, pos]
+        block = [(width,)] * 4 + [(q_rows, width), (kv, width), (kv, width), (width, heads * D), (hidden, width), (width, hidden),
+                                  (q_rows,), (kv,), (kv,), (width,), (hidden,), (width,)]
+        need = (4, 5, 6, 7, 8, 9) if kind else (4, 7, 8, 9)   # the projections
+        rows = [found[TOP + PER_BLOCK * i:TOP + PER_BLOCK * (i + 1)] for i in range(blocks)]
+        if any(f is not None and f[1] != w for f, w in zip(found, want)) or any(r[i] is None for r in rows for i in need) \
+                or any(f is not None and f[1] != w for r in rows for f, w in zip(r, block)) \
+                or (kind and any(f is None or f[2] != "float32" for f in found[6:8])):
+            return
+        ptr = [None if f is None else f[0] for f in found]
+        self.ptrs = (C.c_void_p * max(1, len(ptr) - TOP))(*ptr[TOP:])
+        self.c = _lib.GptModel(kind, code(self.dtype), blocks, width, hidden, heads, kv_heads, vocab, *ptr[:TOP],
+                               C.cast(self.ptrs, C.c_void_p), eps)
+        self.ok = True
 
     def run(self, ids, past=0, position=0, write_pos=0, kv_len=0, max_len=0, k_cache=None, v_cache=None, cache_strides=None,
             last_only=False, softcap=0.0):
@@ -95,24 +103,18 @@ class Plan:
         return logits
 
 
-def plan_of(model, build):
-    """The model's plan, or None when a graph is being recorded, calls are traced one by one, or the
-    model is outside what the call covers. `build(model)` makes a new one."""
+def plan_of(model, describe):
+    """The model's plan as the model is now; None when a graph is being recorded, calls are traced one
+    by one, or the model is outside what the call covers. `describe(model)` walks the model and
+    returns (sizes, arrays) as Plan takes them, or None."""
     if Tensor.build_graph_enabled() or _lib._TRACE:
         return None
+    now = describe(model)
+    if now is None:
+        return None
+    sizes, found = now[0], [None if a is None else (a.ptr, a.shape, a.dtype) for a in now[1]]
     plan = model.__dict__.get("_infer_plan")
-    if plan is None or not plan.valid(model.blocks):
-        plan = build(model)
+    if plan is None or plan.sizes != sizes or plan.found != found:
+        plan = Plan(sizes, found)
         object.__setattr__(model, "_infer_plan", plan)
     return plan if plan.ok else None
-
-
-class NoPlan:
-    """Marks a model that the library call does not cover; looked at again when its blocks change."""
-    ok = False
-
-    def __init__(self, blocks):
-        self.blocks = list(blocks)
-
-    def valid(self, blocks):
-        return len(blocks) == len(self.blocks) and all(a is b for a, b in zip(blocks, self.blocks))

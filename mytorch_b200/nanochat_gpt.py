@@ -178,25 +178,32 @@ def _init_weights(module):      # nanochat_gpt.py:352-369
 
 
 def _plan(model):
-    """Describes the model to the library's whole-model forward (see infer.Plan)."""
+    """What the library's whole-model forward needs to know of the model as it is now (see
+    infer.plan_of); None when it does not cover it."""
     cfg, plain = model.config, infer.plain
-    D = cfg.embed_dim // cfg.num_q_heads
-    ok = plain(model, GPT) and plain(model.embeddings, Embeddings) and plain(model.embeddings.embeddings, nn.Embedding) \
-        and plain(model.lm_head, nn.Linear) and model.lm_head.act_func is None and D in (64, 128)
-    rows = []
+    e, head = model.embeddings, model.lm_head
+    H, Hk, E = cfg.num_q_heads, cfg.num_kv_heads, cfg.embed_dim
+    D = E // H
+    if not (infer.unpatched(_METHODS) and plain(model, GPT) and plain(e, Embeddings) and plain(e.embeddings, nn.Embedding)
+            and plain(head, nn.Linear) and head.act_func is None and D in (64, 128)):
+        return None
+    found = infer.arrays(e.embeddings.weight, None, None, None, head.weight, head.bias) + [model.cos, model.sin]
     for b in model.blocks:
-        ok = ok and plain(b, TransformerBlock) and plain(b.attention, Attention) and plain(b.feedforward, FeedForward)
-        if not ok:
-            break
+        if not plain(b, TransformerBlock):
+            return None
         a, f = b.attention, b.feedforward
-        linears = (a.q_proj, a.k_proj, a.v_proj, a.out_proj, f.intermediate_dense, f.out_proj)
-        ok = all(plain(m, nn.Linear) for m in linears) and [m.act_func for m in linears] == [None] * 4 + ["relu_squared", None] \
-            and (a.num_heads, a.num_kv_heads) == (cfg.num_q_heads, cfg.num_kv_heads)
-        rows.append((None, None, a.q_proj, a.k_proj, a.v_proj, a.out_proj, f.intermediate_dense, f.out_proj))
-    if not ok:
-        return infer.NoPlan(model.blocks)
-    return infer.Plan(model, 1, {"wte": model.embeddings.embeddings, "head": model.lm_head}, model.blocks, rows, cfg.num_q_heads,
-                      cfg.num_kv_heads, cfg.embed_dim * cfg.mlp_ratio, cfg.vocab_size, model.cos, model.sin)
+        if not (plain(a, Attention) and plain(f, FeedForward) and a.num_heads == H and a.num_kv_heads == Hk and a.embed_dim == E
+                and a.head_dim == D):
+            return None
+        q, k, v, out, up, down = a.q_proj, a.k_proj, a.v_proj, a.out_proj, f.intermediate_dense, f.out_proj
+        for m in (q, k, v, out, down):
+            if not (plain(m, nn.Linear) and m.act_func is None):
+                return None
+        if not (plain(up, nn.Linear) and up.act_func == "relu_squared"):
+            return None
+        found += infer.arrays(None, None, None, None, q.weight, k.weight, v.weight, out.weight, up.weight, down.weight,
+                              q.bias, k.bias, v.bias, out.bias, up.bias, down.bias)
+    return (1, len(model.blocks), E, E * cfg.mlp_ratio, H, Hk, cfg.vocab_size, 1e-5), found
 
 
 class GPT(nn.Module):
@@ -231,12 +238,12 @@ class GPT(nn.Module):
         cfg = self.config
         B, T = ids.shape
         past = cache.pos if cache is not None else 0
-        assert past + T <= cfg.max_seq_len, "sequence longer than the rotary table"
+        assert past + T <= min(plan.positions, cfg.max_seq_len), "sequence longer than the rotary table"
         cap = float(cfg.softcap or 0.0) if not self.training else 0.0
         if cache is None:
             return plan.run(ids, last_only=last_only, softcap=cap)
         L, Bc, Hk, S, D = cache.cache_shape
-        if (L, Bc, Hk, D) != (cfg.num_blocks, B, cfg.num_kv_heads, plan.head_dim) or (past and D not in (64, 128)) \
+        if (L, Bc, Hk, D) != (plan.blocks, B, cfg.num_kv_heads, plan.head_dim) \
                 or (cache.k_cache is not None and cache.k_cache.dtype != plan.dtype):
             return None
         assert past + T <= S, "You have filled up your Cache!"
@@ -282,6 +289,12 @@ class GPT(nn.Module):
         loss = F.cross_entropy(logits, target_ids, softcap=self.config.softcap)
         return logits, loss
 
+    def _next_logits(self, feed, cache):
+        """Logits [B, 1 or T, V] after the ids `feed`; the last position is the next token's."""
+        plan = infer.plan_of(self, _plan)
+        out = self._planned(plan, feed, cache, last_only=True) if plan is not None and feed.size else None
+        return self.forward(Tensor(feed), None, cache=cache)[0].data if out is None else out
+
     def generate(self, input_ids, max_new_tokens, temperature=1.0, top_k=None, seed=None):
         """Cached autoregressive sampling for one batch of equally long prompts: the prompt fills a
         KVCache, then one token per step (temperature 0 = arg-max)."""
@@ -294,19 +307,11 @@ class GPT(nn.Module):
         self.eval()
         feed = ids
         with no_grad():
-            plan = infer.plan_of(self, _plan) if ids.size and max_new_tokens > 0 else None
-            if plan is not None and temperature == 0:
-                # the arg-max stays on the device and is the next step's input; one read at the end
-                out, dev = DeviceArray.empty((ids.shape[0], max_new_tokens), "int32"), Tensor(ids).data
-                for i in range(max_new_tokens):
-                    dev = infer.greedy(self._planned(plan, dev, cache, last_only=True), out, i)
-                ids = np.concatenate([ids, out.numpy()], axis=1)
+            if temperature == 0 and max_new_tokens > 0 and ids.size and infer.plan_of(self, _plan) is not None:
+                ids = infer.generate_greedy(self, ids, cache, max_new_tokens)
                 max_new_tokens = 0
             for _ in range(max_new_tokens):
-                if plan is not None:
-                    logits = self._planned(plan, Tensor(feed).data, cache, last_only=True)
-                else:
-                    logits, cache = self.forward(Tensor(feed), None, cache=cache)
+                logits = self._next_logits(Tensor(feed).data, cache)
                 last = logits.numpy()[:, -1, :].astype(np.float64)
                 if temperature == 0:
                     nxt = last.argmax(-1)
@@ -323,3 +328,6 @@ class GPT(nn.Module):
         if was_training:
             self.train()
         return ids
+
+
+_METHODS = infer.methods(GPT, Embeddings, TransformerBlock, Attention, FeedForward, nn.Linear, nn.Embedding)
