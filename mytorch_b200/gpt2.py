@@ -268,9 +268,10 @@ class GPT2(nn.Module):
     def forward(self, x, cache=None):
         """Logits; with a `Cache`, (logits, cache) as in gpt2.py:352-374."""
         from .utils.checkpoint import checkpoint
-        plan = infer.plan_of(self, _plan) if x.data.size else None
-        if plan is not None:
-            out = self._planned(plan, x.data, cache)
+        plan = infer.plan_of(self, _plan)
+        ids = infer.token_ids(x) if plan is not None else None
+        if ids is not None:
+            out = self._planned(plan, ids, cache)
             if out is not None:
                 return Tensor(out) if cache is None else (Tensor(out), cache)
         past_length = cache.get_seq_len() if cache is not None else 0

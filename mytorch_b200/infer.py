@@ -38,6 +38,13 @@ def arrays(*tensors):
     return [None if t is None else t.data for t in tensors]
 
 
+def token_ids(x):
+    """The ids [B, T] on the device; None for what the library call does not take (the layers then
+    accept or refuse it)."""
+    a = x.data if isinstance(x, Tensor) else DeviceArray.from_numpy(x, "int32")
+    return a if a.dtype == "int32" and len(a.shape) == 2 and a.size else None
+
+
 def greedy(logits, ids_out, column):
     """Arg-max of every sequence's last row of logits [B, T, V] into ids_out[:, column] (int32 on the
     device) and as the next step's ids [B, 1]."""

@@ -255,9 +255,10 @@ class GPT(nn.Module):
 
     def forward(self, input_ids, target_ids=None, cache=None):
         B, T = input_ids.shape
-        plan = infer.plan_of(self, _plan) if target_ids is None and B * T else None
-        if plan is not None:
-            out = self._planned(plan, input_ids.data, cache)
+        plan = infer.plan_of(self, _plan) if target_ids is None else None
+        ids = infer.token_ids(input_ids) if plan is not None else None
+        if ids is not None:
+            out = self._planned(plan, ids, cache)
             if out is not None:
                 return (Tensor(out),) if cache is None else (Tensor(out), cache)
         past = cache.pos if cache is not None else 0

@@ -155,3 +155,19 @@ def test_old_arrays_are_not_held(calls):
     del p
     gc.collect()
     assert all(r() is None for r in old)
+
+
+@pytest.mark.parametrize("ids", [np.arange(10).reshape(2, 5), [[1, 2, 3]], np.arange(6, dtype=np.int32).reshape(1, 6)])
+def test_ids_from_the_host(calls, ids):
+    with mt.no_grad():
+        gpt2_model()(ids)
+        if not isinstance(ids, list):
+            nano_model()(ids)
+    assert len(calls) == (1 if isinstance(ids, list) else 2)
+    assert all((p["batch"], p["new_tokens"]) == np.shape(ids) for _, _, p in calls)
+
+
+def test_ids_of_other_kinds_go_to_the_layers(calls):
+    assert infer.token_ids(mt.Tensor(DeviceArray.empty((2, 5), "int64"))) is None
+    assert infer.token_ids(mt.Tensor(DeviceArray.empty((2, 0), "int32"))) is None
+    assert infer.token_ids(mt.Tensor(DeviceArray.empty((5,), "int32"))) is None
