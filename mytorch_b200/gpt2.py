@@ -53,20 +53,19 @@ class Cache:
     def get_seq_len(self, layer_idx=0):
         return min(self._appended[layer_idx], self.max_seq_len)
 
-    def reserve(self, batch, heads, head_dim, dtype):
-        """All layers' rings, allocated together when none of them exists yet. False when the layers
-        do not hold the same number of rows."""
+    def reserve(self, blocks, batch, heads, head_dim, dtype):
+        """All layers' rings, allocated together when none of them exists yet. False when the cache has
+        another number of layers, or its layers do not hold the same number of rows of this shape."""
+        n = len(self.key_cache)
+        if n != blocks or any(a != self._appended[0] for a in self._appended):
+            return False
+        shape = (batch, heads, self.max_seq_len, head_dim)
         if all(k is None for k in self.key_cache):
-            n = len(self.key_cache)
-            rings = DeviceArray.empty((2 * n, batch, heads, self.max_seq_len, head_dim), dtype)
-            ring = lambda i: rings.rows(i, i + 1).reshape(batch, heads, self.max_seq_len, head_dim)
+            rings = DeviceArray.empty((2 * n,) + shape, dtype)
+            ring = lambda i: rings.rows(i, i + 1).reshape(shape)
             self.key_cache = [ring(2 * i) for i in range(n)]
             self.value_cache = [ring(2 * i + 1) for i in range(n)]
-        elif any(k is None for k in self.key_cache):
-            return False
-        kc = self.key_cache[0]
-        assert kc.shape[0] == batch and kc.dtype == dtype, "cache was created for another batch size or dtype"
-        return all(n == self._appended[0] for n in self._appended)
+        return all(r is not None and r.shape == shape and r.dtype == dtype for r in self.key_cache + self.value_cache)
 
     def update(self, k_ptr, v_ptr, strides, batch, heads, n_new, head_dim, dtype, layer_idx):
         """Appends n_new rows read through (ptr, strides) and returns (keys, values, rows held)."""
@@ -254,7 +253,7 @@ class GPT2(nn.Module):
             return plan.run(ids, last_only=last_only)
         cfg, n = self.config, cache.max_seq_len
         D = plan.head_dim
-        if T > n or (past and D not in (64, 128)) or not cache.reserve(B, cfg.num_heads, D, plan.dtype):
+        if T > n or (past and D not in (64, 128)) or not cache.reserve(plan.blocks, B, cfg.num_heads, D, plan.dtype):
             return None
         L = len(cache.key_cache)
         ptrs = C.c_void_p * L

@@ -244,7 +244,7 @@ class GPT(nn.Module):
             return plan.run(ids, last_only=last_only, softcap=cap)
         L, Bc, Hk, S, D = cache.cache_shape
         if (L, Bc, Hk, D) != (plan.blocks, B, cfg.num_kv_heads, plan.head_dim) \
-                or (cache.k_cache is not None and cache.k_cache.dtype != plan.dtype):
+                or any(a is not None and (a.dtype, a.shape) != (plan.dtype, cache.cache_shape) for a in (cache.k_cache, cache.v_cache)):
             return None
         assert past + T <= S, "You have filled up your Cache!"
         k, v = cache.layers(plan.dtype)

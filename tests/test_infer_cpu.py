@@ -171,3 +171,28 @@ def test_ids_of_other_kinds_go_to_the_layers(calls):
     assert infer.token_ids(mt.Tensor(DeviceArray.empty((2, 5), "int64"))) is None
     assert infer.token_ids(mt.Tensor(DeviceArray.empty((2, 0), "int32"))) is None
     assert infer.token_ids(mt.Tensor(DeviceArray.empty((5,), "int32"))) is None
+
+
+def test_caches_of_another_shape_go_to_the_layers(calls):
+    model = gpt2_model()
+    ids = DeviceArray.empty((2, 5), "int32")
+    plan = lambda: infer.plan_of(model, gpt2._plan)
+
+    def cache(**more):
+        return gpt2.Cache(gpt2.GPT2Config(**{**dict(max_seq_len=32, embed_dim=128, num_blocks=2, num_heads=2), **more}))
+    with mt.no_grad():
+        c = cache()
+        assert model._planned(plan(), ids, c) is not None and c.get_seq_len(1) == 5
+        assert model._planned(plan(), DeviceArray.empty((3, 1), "int32"), c) is None         # another batch
+        c.value_cache[1] = DeviceArray.empty((2, 4, 32, 32))
+        assert model._planned(plan(), ids, c) is None
+        for n in (1, 3):                                                                     # the call reads one pointer per block
+            c = cache(num_blocks=n)
+            assert model._planned(plan(), ids, c) is None and c.key_cache == [None] * n
+        assert model._planned(plan(), ids, cache(max_seq_len=4)) is None
+        with pytest.raises(AssertionError, match="position table"):
+            model._planned(plan(), DeviceArray.empty((1, 33), "int32"), None)
+        nano = nano_model()
+        k = nanochat_gpt.KVCache(2, 1, 32, 64, 2)
+        k.k_cache = DeviceArray.empty((2, 2, 1, 16, 64))
+        assert nano._planned(infer.plan_of(nano, nanochat_gpt._plan), ids, k) is None
