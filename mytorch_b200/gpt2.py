@@ -200,7 +200,7 @@ def _plan(model):
         return None
     H, E = cfg.num_heads, cfg.embed_dim
     eps = {lnf.eps}
-    found = infer.arrays(e.char_embeddings.weight, e.position_embeddings.weight, lnf.weight, lnf.bias, head.weight, head.bias) + [None, None]
+    found = [e.char_embeddings.weight, e.position_embeddings.weight, lnf.weight, lnf.bias, head.weight, head.bias, None, None]
     for b in model.blocks:
         if not plain(b, TransformerBlock):
             return None
@@ -216,11 +216,11 @@ def _plan(model):
             if not (plain(drop, nn.Dropout) and drop.p == 0.0):
                 return None
         eps.update((n1.eps, n2.eps))
-        found += infer.arrays(n1.weight, n1.bias, n2.weight, n2.bias, qkv.weight, None, None, out.weight, up.weight, down.weight,
-                              qkv.bias, None, None, out.bias, up.bias, down.bias)
+        found += [n1.weight, n1.bias, n2.weight, n2.bias, qkv.weight, None, None, out.weight, up.weight, down.weight,
+                  qkv.bias, None, None, out.bias, up.bias, down.bias]
     if len(eps) > 1:
         return None
-    return (0, len(model.blocks), E, E * cfg.mlp_ratio, H, H, cfg.vocab_size, eps.pop()), found
+    return (0, E, E * cfg.mlp_ratio, H, H, cfg.vocab_size, eps.pop()), found, _METHODS
 
 
 class GPT2(nn.Module):

@@ -187,7 +187,7 @@ def _plan(model):
     if not (infer.unpatched(_METHODS) and plain(model, GPT) and plain(e, Embeddings) and plain(e.embeddings, nn.Embedding)
             and plain(head, nn.Linear) and head.act_func is None and D in (64, 128)):
         return None
-    found = infer.arrays(e.embeddings.weight, None, None, None, head.weight, head.bias) + [model.cos, model.sin]
+    found = [e.embeddings.weight, None, None, None, head.weight, head.bias, model.cos, model.sin]
     for b in model.blocks:
         if not plain(b, TransformerBlock):
             return None
@@ -201,9 +201,9 @@ def _plan(model):
                 return None
         if not (plain(up, nn.Linear) and up.act_func == "relu_squared"):
             return None
-        found += infer.arrays(None, None, None, None, q.weight, k.weight, v.weight, out.weight, up.weight, down.weight,
-                              q.bias, k.bias, v.bias, out.bias, up.bias, down.bias)
-    return (1, len(model.blocks), E, E * cfg.mlp_ratio, H, Hk, cfg.vocab_size, 1e-5), found
+        found += [None, None, None, None, q.weight, k.weight, v.weight, out.weight, up.weight, down.weight,
+                  q.bias, k.bias, v.bias, out.bias, up.bias, down.bias]
+    return (1, E, E * cfg.mlp_ratio, H, Hk, cfg.vocab_size, 1e-5), found, _METHODS
 
 
 class GPT(nn.Module):

@@ -5,6 +5,7 @@ RMSNorm, GELU, ReLUSquared, Dropout (p = 0), CrossEntropyLoss, ModuleList,
 Sequential (mytorch/nn/modules/**). Parameters are drawn on the host with the
 NumPy global generator, as in mytorch/nn/initializations.py:44-56, so that a
 seed gives the same weights as the reference."""
+import itertools
 import math
 
 import numpy as np
@@ -20,7 +21,14 @@ def Parameter(array):
     return t
 
 
+_edit = itertools.count(1)
+
+
 class Module:
+    # A new number after every assignment to or deletion of an attribute of any module: what was derived
+    # from a model's structure is still good while it stands (infer.plan_of).
+    edits = 0
+
     def __init__(self):
         object.__setattr__(self, "_modules", {})
         object.__setattr__(self, "_params", {})
@@ -36,10 +44,16 @@ class Module:
         elif name in self._params and value is None:
             del self._params[name]
         object.__setattr__(self, name, value)
+        Module.edits = next(_edit)
+
+    def __delattr__(self, name):
+        object.__delattr__(self, name)
+        Module.edits = next(_edit)
 
     def register_buffer(self, name, tensor, persistent=True):
         self._buffers[name] = (tensor, persistent)
         object.__setattr__(self, name, tensor)
+        Module.edits = next(_edit)
 
     def __call__(self, *a, **k):
         return self.forward(*a, **k)

@@ -83,11 +83,14 @@ GPT2_OUTSIDE = {
     "final norm's size": lambda m: setattr(m.final_layer_norm.bias, "data", DeviceArray.empty((64,))),
     "bias's size": lambda m: setattr(m.blocks[0].attention.out_proj, "bias", mt.Tensor(DeviceArray.empty((64,)), requires_grad=True)),
     "heads": lambda m: setattr(m.blocks[0].attention, "num_heads", 1),
+    "config": lambda m: setattr(m.config, "num_heads", 4),
+    "own class": lambda m: setattr(m.blocks[0].attention, "__class__", type("Mine", (gpt2.Attention,), {})),
 }
 NANO_EDITS = {
     "key projection": lambda m: setattr(m.blocks[1].attention, "k_proj", weight(64, 128)),
     "head": lambda m: setattr(m, "lm_head", weight(96, 128)),
     "embeddings": lambda m: setattr(m.embeddings, "embeddings", nn.Embedding(96, 128)),
+    "buffers": lambda m: m.register_buffer("cos", DeviceArray.empty((32, 64))),
     "rotary tables": lambda m: (setattr(m, "cos", DeviceArray.empty((32, 64))), setattr(m, "sin", DeviceArray.empty((32, 64)))),
 }
 NANO_OUTSIDE = {
@@ -155,6 +158,17 @@ def test_old_arrays_are_not_held(calls):
     del p
     gc.collect()
     assert all(r() is None for r in old)
+
+
+def test_a_plan_is_kept_while_nothing_changes(calls):
+    model = gpt2_model()
+    assert forward(model)
+    plan = model._infer_plan
+    model.train()
+    model.eval()
+    assert forward(model) and model._infer_plan is plan
+    nn.Linear(1, 1).act_func = None           # any module's edit: looked at again
+    assert forward(model) and model._infer_plan is not plan
 
 
 @pytest.mark.parametrize("ids", [np.arange(10).reshape(2, 5), [[1, 2, 3]], np.arange(6, dtype=np.int32).reshape(1, 6)])
