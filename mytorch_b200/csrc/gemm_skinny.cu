@@ -405,29 +405,10 @@ skinny_kernel(const SkinnyParams p) {
   if (threadIdx.x == 0 && *abort_flag && p.flag) atomicMax(p.flag, 105);   // a bounded wait expired
 }
 
-bool skinny_supported(const SkinnyArgs& a) {
-  const bool f32 = a.dtype == MT_F32;
-  const int vec = f32 ? 4 : 8;
-  if (a.M < 1 || a.M > kSkinnyMaxRows) return false;
-  if (a.K < vec || a.K % vec || a.ldx % vec || a.ldw % vec || !aligned16(a.x)) return false;
-  for (int i = 0; i < a.nseg; ++i) {
-    if (!aligned16(a.w[i]) || a.n[i] < 1) return false;
-    if (a.nseg > 1 && a.n[i] % 8) return false;            // a group of rows lies in one segment
-  }
-  if (a.norm && ((a.gamma && !aligned16(a.gamma)) || (a.beta && !aligned16(a.beta)))) return false;
-  if (a.norm && !f32 && a.M > 32) return false;
-  // the rows of x of one block have to fit shared memory beside a ring of weights
-  const int64_t rows = f32 ? (a.M < 16 ? a.M : 16) : a.M, es = f32 ? 4 : 2;
-  const int64_t kc = a.norm ? a.K : (a.K + 7) / 8;
-  return rows * kc * es <= 100 * 1024 && a.K <= 32768;
-}
-
 constexpr size_t kSkSmemMax = 226 * 1024;
 
-struct SkinnyShape { int gr, blocks, cluster, kc, its, rounds, ring, x_bytes, nb_bytes; size_t smem; double cost; };
-
 // How a product runs with gr groups per round, K split over `cluster` blocks and per_sm blocks resident
-// on an SM; cost in cycles of the busiest SM.
+// on an SM.
 template <typename T>
 static SkinnyShape skinny_shape(const SkinnyArgs& a, int N, int mv, int gr, int cluster, int per_sm) {
   constexpr int R = SkinnyGroup<T>::rows;
@@ -480,7 +461,6 @@ static int launch_skinny(const SkinnyArgs& a, SkinnyParams& p, const SkinnyShape
     MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     if (dev >= 0 && dev < 16) ready[dev].store(true, std::memory_order_release);
   }
-  MT_REQUIRE(s.cost < 1e30, "skinny gemm: %zu bytes of shared memory", s.smem);
   p.kc = s.kc; p.its = s.its; p.rounds = s.rounds; p.ring = s.ring;
   p.x_bytes = s.x_bytes; p.nb_bytes = s.nb_bytes;
   p.whole_rows = s.cluster == 1 && a.ldw == a.K;
@@ -503,32 +483,72 @@ static int launch_skinny(const SkinnyArgs& a, SkinnyParams& p, const SkinnyShape
   return MT_OK;
 }
 
+template <typename T, int MV> constexpr int skinny_most_groups() { return sizeof(T) == 2 ? (MV <= 32 ? 5 : 3) : 4; }
+
 template <typename T, int MV>
-static int launch_skinny_shape(const SkinnyArgs& a, SkinnyParams& p, cudaStream_t st) {
-  constexpr bool kHalf = sizeof(T) == 2;
-  constexpr int GM = kHalf ? (MV <= 32 ? 5 : 3) : 4;
+static SkinnyShape best_shape(const SkinnyArgs& a, int N) {
   SkinnyShape best{};
   best.cost = 1e30;
   for (int cluster = 1; cluster <= 8; cluster *= 2) {
     if (cluster > 1 && (a.norm || a.K < 512 * cluster)) break;        // a norm needs whole rows
-    for (int gr = 1; gr <= GM; ++gr) {
-      if (!kHalf && gr == 3) continue;
+    for (int gr = 1; gr <= skinny_most_groups<T, MV>(); ++gr) {
+      if (sizeof(T) == 4 && gr == 3) continue;
       for (int per_sm = 1; per_sm <= 2; ++per_sm) {
-        const SkinnyShape s = skinny_shape<T>(a, p.N, MV, gr, cluster, per_sm);
+        const SkinnyShape s = skinny_shape<T>(a, N, MV, gr, cluster, per_sm);
         if (s.cost < best.cost) best = s;
       }
     }
   }
-  switch (best.gr) {
-    case 1: return launch_skinny<T, MV, 1>(a, p, best, st);
-    case 2: return launch_skinny<T, MV, 2>(a, p, best, st);
-    case 3: return launch_skinny<T, MV, kHalf ? 3 : 1>(a, p, best, st);
-    case 4: return launch_skinny<T, MV, GM >= 4 ? 4 : 1>(a, p, best, st);
-    default: return launch_skinny<T, MV, GM >= 5 ? 5 : 1>(a, p, best, st);
+  return best;
+}
+
+template <typename T, int MV>
+static int launch_skinny_shape(const SkinnyArgs& a, SkinnyParams& p, const SkinnyShape& s, cudaStream_t st) {
+  constexpr bool kHalf = sizeof(T) == 2;
+  constexpr int GM = skinny_most_groups<T, MV>();
+  switch (s.gr) {
+    case 1: return launch_skinny<T, MV, 1>(a, p, s, st);
+    case 2: return launch_skinny<T, MV, 2>(a, p, s, st);
+    case 3: return launch_skinny<T, MV, kHalf ? 3 : 1>(a, p, s, st);
+    case 4: return launch_skinny<T, MV, GM >= 4 ? 4 : 1>(a, p, s, st);
+    default: return launch_skinny<T, MV, GM >= 5 ? 5 : 1>(a, p, s, st);
   }
 }
 
-int skinny_gemm(const SkinnyArgs& a, cudaStream_t st) {
+// FN<T, MV>(...) with the rows of x that a block covers.
+#define MT_SKINNY_ROWS(a, FN, ...)                                                                                    \
+  ((a).dtype == MT_F32   ? ((a).M == 1   ? FN<float, 1>(__VA_ARGS__)                                                  \
+                            : (a).M == 2 ? FN<float, 2>(__VA_ARGS__)                                                  \
+                            : (a).M <= 4 ? FN<float, 4>(__VA_ARGS__)                                                  \
+                            : (a).M <= 8 ? FN<float, 8>(__VA_ARGS__) : FN<float, 16>(__VA_ARGS__))                    \
+   : (a).dtype == MT_F16 ? ((a).M <= 16   ? FN<__half, 16>(__VA_ARGS__)                                               \
+                            : (a).M <= 32 ? FN<__half, 32>(__VA_ARGS__) : FN<__half, 64>(__VA_ARGS__))                \
+                         : ((a).M <= 16   ? FN<__nv_bfloat16, 16>(__VA_ARGS__)                                        \
+                            : (a).M <= 32 ? FN<__nv_bfloat16, 32>(__VA_ARGS__) : FN<__nv_bfloat16, 64>(__VA_ARGS__)))
+
+bool skinny_fits(const SkinnyArgs& a, SkinnyShape& shape) {
+  const bool f32 = a.dtype == MT_F32;
+  const int vec = f32 ? 4 : 8;
+  if (a.M < 1 || a.M > kSkinnyMaxRows) return false;
+  if (a.K < vec || a.K % vec || a.ldx % vec || a.ldw % vec || !aligned16(a.x)) return false;
+  for (int i = 0; i < a.nseg; ++i) {
+    if (!aligned16(a.w[i]) || a.n[i] < 1) return false;
+    if (a.nseg > 1 && a.n[i] % 8) return false;            // a group of rows lies in one segment
+  }
+  if (a.norm && ((a.gamma && !aligned16(a.gamma)) || (a.beta && !aligned16(a.beta)))) return false;
+  if (a.norm && !f32 && a.M > 32) return false;
+  // The rows of x of one block have to fit shared memory beside a ring of weights: a quick bound here; the launch
+  // shapes have the last word (a norm keeps K whole: eight rows in half types end near K = 4200).
+  const int64_t rows = f32 ? (a.M < 16 ? a.M : 16) : a.M, es = f32 ? 4 : 2;
+  const int64_t kc = a.norm ? a.K : (a.K + 7) / 8;
+  if (rows * kc * es > 100 * 1024 || a.K > 32768) return false;
+  int N = 0;
+  for (int i = 0; i < a.nseg; ++i) N += a.n[i];
+  shape = MT_SKINNY_ROWS(a, best_shape, a, N);
+  return shape.cost < 1e30;
+}
+
+int skinny_gemm(const SkinnyArgs& a, const SkinnyShape& shape, cudaStream_t st) {
   SkinnyParams p{};
   p.x = a.x; p.ldx = a.ldx; p.M = a.M; p.K = a.K;
   for (int i = 0; i < 3; ++i) { p.w[i] = a.w[i]; p.bias[i] = a.bias[i]; }
@@ -542,17 +562,7 @@ int skinny_gemm(const SkinnyArgs& a, cudaStream_t st) {
   p.early = a.early_weights;
   p.norm = a.norm;
   p.flag = device_flag_ptr();
-  if (a.dtype != MT_F32) {
-    const bool f16 = a.dtype == MT_F16;
-    if (a.M <= 16) return f16 ? launch_skinny_shape<__half, 16>(a, p, st) : launch_skinny_shape<__nv_bfloat16, 16>(a, p, st);
-    if (a.M <= 32) return f16 ? launch_skinny_shape<__half, 32>(a, p, st) : launch_skinny_shape<__nv_bfloat16, 32>(a, p, st);
-    return f16 ? launch_skinny_shape<__half, 64>(a, p, st) : launch_skinny_shape<__nv_bfloat16, 64>(a, p, st);
-  }
-  if (a.M == 1) return launch_skinny_shape<float, 1>(a, p, st);
-  if (a.M == 2) return launch_skinny_shape<float, 2>(a, p, st);
-  if (a.M <= 4) return launch_skinny_shape<float, 4>(a, p, st);
-  if (a.M <= 8) return launch_skinny_shape<float, 8>(a, p, st);
-  return launch_skinny_shape<float, 16>(a, p, st);
+  return MT_SKINNY_ROWS(a, launch_skinny_shape, a, p, shape, st);
 }
 
 }  // namespace mt

@@ -996,9 +996,10 @@ int mt_gemm_ex(const void* A, const void* B, void* C, void* preact, const void* 
     a.x = A; a.ldx = lda; a.M = (int)M; a.K = (int)K; a.dtype = in_dtype;
     a.w[0] = B; a.bias[0] = bias; a.n[0] = (int)N; a.ldw = ldb;
     a.out = C; a.ldo = ldc; a.residual = aux; a.act = act & 0xff;
-    if (N < (1ll << 31) && K < (1ll << 31) && skinny_supported(a)) {
+    SkinnyShape shape;
+    if (N < (1ll << 31) && K < (1ll << 31) && skinny_fits(a, shape)) {
       ProfScope prof(PROF_GEMM, st, 2.0 * (double)M * (double)N * (double)K);
-      return skinny_gemm(a, st);
+      return skinny_gemm(a, shape, st);
     }
   }
   if (!g_force_simt && gemm_tc_supported(g)) return gemm_tc(g, st);

@@ -31,7 +31,10 @@ struct SkinnyArgs {
 };
 
 constexpr int kSkinnyMaxRows = 64;       // half: four 16-row MMA tiles; fp32: chunks of up to 16 rows per block
-bool skinny_supported(const SkinnyArgs& a);
-int skinny_gemm(const SkinnyArgs& a, cudaStream_t st);
+
+// How a product is laid out over the chip (gemm_skinny.cu); cost in cycles of the busiest SM.
+struct SkinnyShape { int gr, blocks, cluster, kc, its, rounds, ring, x_bytes, nb_bytes; size_t smem; double cost; };
+bool skinny_fits(const SkinnyArgs& a, SkinnyShape& shape);      // whether the product can be taken, and how
+int skinny_gemm(const SkinnyArgs& a, const SkinnyShape& shape, cudaStream_t st);
 
 }  // namespace mt

@@ -107,6 +107,25 @@ def test_whole_model_forward_matches_the_ops(mt, monkeypatch, dtype, kind, heads
     no_device_flag(mt)
 
 
+# Wide rows behind a norm: sizes whose rows, weights and sums no launch of the folded product holds (they take the norm and
+# the product one after the other), and the last that one holds.
+@pytest.mark.parametrize("dtype,width,B", [("float16", 4096, 10), ("bfloat16", 4096, 12), ("float16", 8192, 1), ("float32", 4096, 5),
+                                           ("float32", 8192, 1), ("float16", 4096, 4)])
+def test_wide_norm_and_head(mt, monkeypatch, dtype, width, B):
+    from mytorch_b200 import infer
+    from mytorch_b200.gpt2 import GPT2, GPT2Config
+    model = GPT2(GPT2Config(vocab_size=3000, max_seq_len=2, embed_dim=width, num_blocks=0, num_heads=width // 128))
+    for p in model.parameters():
+        p.astype(dtype)
+    ids = mt.Tensor(np.arange(B, dtype=np.int32)[:, None])
+    with mt.no_grad():
+        got = model(ids).numpy()
+        assert model._infer_plan.ok
+        monkeypatch.setattr(infer, "plan_of", lambda m, b: None)
+        close(got, model(ids).numpy(), 2 * TOL[dtype], "logits")
+    no_device_flag(mt)
+
+
 def test_plans_follow_the_weights(mt):
     """Replaced, cast or reloaded weights are used by the next forward."""
     model = models(mt, "gpt2", "float32", 2, 2, 64, False)
