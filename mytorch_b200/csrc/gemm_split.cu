@@ -6,10 +6,14 @@
 // below 2^-26 |x|), a half value is copied. `gemm_split_kernel` then multiplies plane by plane:
 //   fp32: l.h + h.l + m.m + m.h + h.m + h.h, smallest first; the products left out (m.l, l.m, l.l) are below
 //   2^-25 of a term. Every bf16 product is exact in the fp32 accumulator.
-// The accumulator in tensor memory is not kept over all of K: after each chunk of K the epilogue warps
-// add it to fp32 registers (round to nearest) while the next chunk goes to the other accumulator.
-// Relative error against 64 bits (2-norm, normal data): K = 256 8.6e-8 (FMA chain 2.9e-7), 768 1.0e-7 (5.0e-7),
-// 4096 1.1e-7 (1.1e-6), 8192 2.2e-7 (1.6e-6).
+// The accumulator in tensor memory is not kept over all of K, for its additions cut off instead of rounding:
+// after each chunk of K the epilogue warps add it to fp32 registers (round to nearest) while the next chunk goes to
+// the other accumulator. The chunk is chosen so that the sum is no further from 64 bits than a chain of
+// fp32 FMAs (relative error, 2-norm; in brackets the chain's):
+//   fp32, every 64 of K:  K = 16 4.8e-8 (7.4e-8), 256 8.8e-8 (2.9e-7), 3072 1.2e-7 (9.9e-7), 131072 3.0e-7 (6.5e-6) of
+//   normal values; of values in [0, 1) 5.2e-8 (6.2e-8), 8.7e-8 (2.2e-7), 9.7e-8 (7.8e-7), 1.3e-7 (6.9e-6).
+//   fp16 in [0, 1), the worst case of the half types, every 64 of K 1.9e-7, 128 4.7e-7, 256 1.15e-6, 512 2.65e-6 whatever
+//   K is; the chain 1.4e-8 sqrt(K), which is smaller below K = 200.
 //
 // Persistent. A slot of a CTA's ring holds 128 rows of one plane of A and of B (2 x 16 KB), a 64-deep slice of fp32
 // operands three slots. A CTA pair (cta_group::2) works on a 256 x 256 tile: the 24 MMAs of a slice last 3072 tensor
@@ -282,8 +286,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (n < P.N) {
             const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
             const int rows = (int)min((int64_t)32, P.M - m0);
-            const bool plain = !P.preact && !P.act && !P.aux_mode && !P.accumulate && P.out_dtype == MT_F32;
-            float* const c = (float*)P.C + m0 * P.ldc + n;
+            const bool plain = !P.preact && !P.act && !P.aux_mode && !P.accumulate;
             for (int r0 = 0; r0 < rows; r0 += 8) {
               float v[8];
               bool fine = plain && r0 + 8 <= rows;
@@ -294,7 +297,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
               }
               if (fine) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) c[(r0 + u) * P.ldc] = P.alpha * v[u] + bias;
+                for (int u = 0; u < 8; ++u) store_typed(P.C, (m0 + r0 + u) * P.ldc + n, P.out_dtype, P.alpha * v[u] + bias);
               } else {
                 // (kept small: eight copies of it in a row ran 15 % slower, on instruction fetches)
 #pragma unroll 2
@@ -420,7 +423,7 @@ prepare_kernel(const PrepareJob a, const PrepareJob b) {
 constexpr double kSplitMinUs = 30.0;
 
 bool gemm_split_supported(const GemmArgs& g) {
-  if (g.M < 16 || g.N < 16 || g.K < 16) return false;
+  if (g.M < 16 || g.N < 16 || g.K < (g.in_dtype == MT_F32 ? 16 : 256)) return false;   // (half, K = 91: error 1.56e-7, FMA chain 1.46e-7)
   if (g.M >= (1ll << 30) || g.N >= (1ll << 30) || g.K > (1ll << 17)) return false;   // (K: the time a row of plain dot products may take)
   const double tiles = (double)((g.M + 63) / 64) * (double)((g.N + 63) / 64) / (0.87 * sm_count());
   return 8.0 + 0.05 * (double)g.K * (tiles > 1.0 ? tiles : 1.0) >= kSplitMinUs;
@@ -488,14 +491,6 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
     else MT_CHECK_CUDA(launch_overlapped(prepare_kernel<false>, grid, dim3(256), 0, st, job[0], job[1]));
     count_launch();
   }
-  // A half output without an activation: its rounding hides how the long sum is kept, and the CTA-pair kernel is the
-  // faster one on the rewritten operands (bf16 3885 x 50257 -> 768: 719 -> 431 us). With an activation it is not taken: its tanh is an approximation.
-  if (!f32 && g.out_dtype != MT_F32 && (g.act & 0xff) == MT_ACT_NONE && !g.preact && g.aux_mode != 2) {
-    GemmArgs t = g;
-    if (job[0].units) { t.A = job[0].dst; t.lda = job[0].pitch; }
-    if (job[1].units) { t.B = job[1].dst; t.ldb = job[1].pitch; }
-    return gemm_tc(t, st);
-  }
   CUtensorMap map[2];
   const bool mn[2] = {g.trans_a != 0, g.trans_b == 0};
   for (int i = 0; i < 2; ++i) {
@@ -514,7 +509,9 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
   P.trans_a = g.trans_a; P.trans_b = g.trans_b; P.in_dtype = g.in_dtype; P.out_dtype = g.out_dtype;
   P.act = g.act; P.aux_mode = g.aux_mode; P.accumulate = g.accumulate; P.alpha = g.alpha;
   P.kb_total = (int)((g.K + kSpK - 1) / kSpK);
-  P.chunk = f32 || g.out_dtype == MT_F32 ? 1 : 4;      // a half output's own rounding hides what four slices lose
+  // Slices that stay in tensor memory: the error grows with them, the FMA chain's with sqrt(K), and the epilogue's additions
+  // cost time (3885 x 50257 -> 768: one slice 700 us, two 585, four 515, eight 479).
+  P.chunk = f32 || g.K < 2048 ? 1 : g.K < 12288 ? 2 : g.K < 49152 ? 4 : 8;
   P.flag = device_flag_ptr();
   // Neighbouring tiles share the larger operand's panel unless it fits the L2 anyway.
   P.n_fast = g.M > g.N ? 1 : 0;

@@ -58,6 +58,37 @@ def test_half_products_with_odd_pitches(mt, dtype, ta, tb, M, N, K):
     no_device_flag(mt)
 
 
+def errors(mt, A, B, want, out_dtype):
+    """Relative errors (2-norm) of A B^T as dispatched and as a chain of fp32 FMAs."""
+    out = []
+    for simt in (0, 1):
+        mt._lib.gemm_force_simt(simt)
+        try:
+            got = mt.fused_ops.gemm(A, B, trans_b=True, out_dtype=out_dtype).numpy().astype(np.float64)
+        finally:
+            mt._lib.gemm_force_simt(0)
+        out.append(np.linalg.norm(got - want) / np.linalg.norm(want))
+    return out
+
+
+# both sides of every length that the sum stays in tensor memory, and of the shortest K that goes there
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("K", [91, 255, 257, 2047, 2049, 12287, 12289, 49151, 50257])
+def test_half_sums_are_no_less_exact_than_an_fp32_chain(mt, dtype, K):
+    """Values of one sign: what the tensor cores cut off adds up in one direction. (A half output adds its own rounding, in
+    which the sums' difference shows as less than 1 %.)"""
+    n = 1000 if K < 3000 else 200
+    r = np.random.default_rng(K)
+    a, b = rnd(r.random((n, K)), dtype), rnd(r.random((n, K)) / np.sqrt(K), dtype)
+    A, B = dev(mt, a, dtype), dev(mt, b, dtype)
+    want = a.astype(np.float64) @ b.T.astype(np.float64)
+    fast, chain = errors(mt, A, B, want, "float32")
+    assert fast <= chain, (fast, chain)
+    fast, chain = errors(mt, A, B, want, dtype)
+    assert fast <= 1.01 * chain, (fast, chain)
+    no_device_flag(mt)
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000)])          # one CTA per tile, a cluster per tile
 def test_epilogues_match_the_cuda_core_kernel(mt, M, N, K):
     F = mt.fused_ops
