@@ -2,8 +2,8 @@
 // chain of fp32 FMAs: fp32 matrices, and half matrices whose pointers or pitches TMA cannot address.
 //
 // Two launches. `prepare_kernel` rewrites the operands with a 16-byte pitch: an fp32 value x becomes three
-// bf16 planes h + m + l = x (8 significant bits each, rounded to nearest, so what is left over is
-// below 2^-26 |x|), a half value is copied. `gemm_split_kernel` then multiplies plane by plane:
+// bf16 planes h + m + l = 2^24 x (8 significant bits each, rounded to nearest: exact; the factor keeps the planes of
+// the smallest fp32 values among bf16's normal numbers, and the sums are multiplied by 2^-48), a half value is copied. `gemm_split_kernel` then multiplies plane by plane:
 //   fp32: l.h + h.l + m.m + m.h + h.m + h.h, smallest first; the products left out (m.l, l.m, l.l) are below
 //   2^-25 of a term. Every bf16 product is exact in the fp32 accumulator.
 // The accumulator in tensor memory is not kept over all of K, for its additions cut off instead of rounding:
@@ -24,9 +24,8 @@
 // fp32: 8192 x 768 -> 3072 1414 -> 202 us, its weight gradient 1529 -> 260, 4096 x 256 -> 1024 102 -> 25, 256 x 4096 x 256
 // 209 -> 25; bf16 with odd pitches and fp32 output: 50257 x 3885 -> 768 12345 -> 526 us.
 //
-// A result that is not finite (an operand is, or |x| > 3.39e38 rounds to bf16 infinity) is computed
+// A result that is not finite (an operand is, or one is above 2^103, or a sum above 2^79) is computed
 // again as a plain fp32 dot product, so infinities and NaNs come out as fp32 arithmetic gives them.
-// Operands below 2^-108 lose their last plane to bf16's exponent range.
 #include "gemm.cuh"
 #include "sm100.cuh"
 #include "prof.cuh"
@@ -48,6 +47,8 @@ constexpr int kSpStage = 32 * 33 * 4;                // an epilogue warp's 32 x 
 constexpr int kSpSmem = kSpSlots * kSpSlot + kSpEpiWarps * kSpStage + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int kSpPitch = kSpN + 1;                   // row pitch (floats) of the sums a cluster exchanges
 static_assert(kSpM * kSpPitch * 4 <= kSpSlots * kSpSlot, "a tile's sums fit the ring");
+
+constexpr float kSpScale = 16777216.f, kSpUnscale = 1.f / (kSpScale * kSpScale);     // exact
 
 struct SplitParams {
   const void* A; const void* B; void* C; void* preact; const void* bias; const void* aux;
@@ -80,7 +81,7 @@ static __device__ __noinline__ float split_dot(const SplitParams& P, int64_t m, 
 // Everything behind the sum of one output; aux and old are what its aux operand and C hold (0 where not read).
 template <bool F32>
 __device__ __forceinline__ void split_finish(const SplitParams& P, float v, float bias, float aux, float old, int64_t m, int64_t n) {
-  if (F32 && !(fabsf(v) <= 3.402823466e38f)) v = split_dot(P, m, n);
+  if (F32) v = fabsf(v) <= 3.402823466e38f ? v * kSpUnscale : split_dot(P, m, n);
   v = P.alpha * v + bias;
   const int64_t off = m * P.ldc + n;
   if (P.preact) store_typed(P.preact, off, P.out_dtype, (P.act & kActStoreGrad) ? act_grad(v, P.act) : v);
@@ -297,7 +298,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
               }
               if (fine) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) store_typed(P.C, (m0 + r0 + u) * P.ldc + n, P.out_dtype, P.alpha * v[u] + bias);
+                for (int u = 0; u < 8; ++u) store_typed(P.C, (m0 + r0 + u) * P.ldc + n, P.out_dtype, P.alpha * (F32 ? v[u] * kSpUnscale : v[u]) + bias);
               } else {
                 // (kept small: eight copies of it in a row ran 15 % slower, on instruction fetches)
 #pragma unroll 2
@@ -397,8 +398,9 @@ prepare_kernel(const PrepareJob a, const PrepareJob b) {
       Vec16<__nv_bfloat16> h, m, l;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        h.e[e] = __float2bfloat16_rn(x[e]);
-        const float r = x[e] - __bfloat162float(h.e[e]);       // exact
+        const float v = x[e] * kSpScale;
+        h.e[e] = __float2bfloat16_rn(v);
+        const float r = v - __bfloat162float(h.e[e]);          // exact
         m.e[e] = __float2bfloat16_rn(r);
         l.e[e] = __float2bfloat16_rn(r - __bfloat162float(m.e[e]));
       }

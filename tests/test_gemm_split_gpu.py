@@ -89,6 +89,19 @@ def test_half_sums_are_no_less_exact_than_an_fp32_chain(mt, dtype, K):
     no_device_flag(mt)
 
 
+# Magnitudes down to fp32's subnormals, whose last bits are what is left of a value; both one CTA per tile and a cluster
+@pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000), (2100, 1000, 64)])
+@pytest.mark.parametrize("ea,eb", [(-100, 0), (-112, 0), (-118, 10), (-126, 20), (-135, 60), (-147, 90), (90, -100), (60, 10)])
+def test_small_and_large_magnitudes(mt, M, N, K, ea, eb):
+    r = np.random.default_rng(K + 200 - ea)
+    a = (r.standard_normal((M, K)) * 2.0 ** ea).astype(np.float32)
+    b = (r.standard_normal((N, K)) * 2.0 ** eb).astype(np.float32)
+    want, size = product(a, b, 0, 1)
+    got = mt.fused_ops.gemm(dev(mt, a, "float32"), dev(mt, b, "float32"), trans_b=True).numpy()
+    assert (np.abs(got - want) <= bound(K) * size + 2.0 ** -149).all(), (np.abs(got - want) / size).max() / bound(K)
+    no_device_flag(mt)
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000)])          # one CTA per tile, a cluster per tile
 def test_epilogues_match_the_cuda_core_kernel(mt, M, N, K):
     F = mt.fused_ops
