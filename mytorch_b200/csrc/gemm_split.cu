@@ -24,8 +24,9 @@
 // fp32: 8192 x 768 -> 3072 1414 -> 202 us, its weight gradient 1529 -> 260, 4096 x 256 -> 1024 102 -> 25, 256 x 4096 x 256
 // 209 -> 25; bf16 with odd pitches and fp32 output: 50257 x 3885 -> 768 12345 -> 526 us.
 //
-// A result that is not finite (an operand is, or one is above 2^103, or a sum above 2^79) is computed
-// again as a plain fp32 dot product, so infinities and NaNs come out as fp32 arithmetic gives them.
+// A sum that is not finite (an operand is, or one is above 2^103, or the result above 2^79) is computed again as a plain
+// chain of fp32 FMAs, so infinities and NaNs come out as fp32 arithmetic gives them. The epilogue only leaves such 32 x 32
+// pieces out and marks them; they are made up after the CTA's last tile, when no role waits for another any more.
 #include "gemm.cuh"
 #include "sm100.cuh"
 #include "prof.cuh"
@@ -56,6 +57,7 @@ struct SplitParams {
   int trans_a, trans_b, in_dtype, out_dtype, act, aux_mode, accumulate;
   float alpha;
   int tiles_m, tiles_n, n_fast, csize, kb_total, kb_per_rank, chunk;
+  uint8_t* left_out;        // fp32, K not split: [tile][CTA][epilogue warp] the pieces (bit = 32 columns) that are made up at the end
   int* flag;
 };
 
@@ -68,20 +70,10 @@ __device__ __forceinline__ void store_typed(void* p, int64_t i, int dt, float v)
   else ((__nv_bfloat16*)p)[i] = __float2bfloat16_rn(v);
 }
 
-// The dot product of one output in plain fp32.
-static __device__ __noinline__ float split_dot(const SplitParams& P, int64_t m, int64_t n) {
-  const float* a = (const float*)P.A + (P.trans_a ? m : m * P.lda);
-  const float* b = (const float*)P.B + (P.trans_b ? n * P.ldb : n);
-  const int64_t sa = P.trans_a ? P.lda : 1, sb = P.trans_b ? 1 : P.ldb;
-  float v = 0.f;
-  for (int64_t k = 0; k < P.K; ++k) v = fmaf(a[k * sa], b[k * sb], v);
-  return v;
-}
+__device__ __forceinline__ bool split_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
 // Everything behind the sum of one output; aux and old are what its aux operand and C hold (0 where not read).
-template <bool F32>
 __device__ __forceinline__ void split_finish(const SplitParams& P, float v, float bias, float aux, float old, int64_t m, int64_t n) {
-  if (F32) v = fabsf(v) <= 3.402823466e38f ? v * kSpUnscale : split_dot(P, m, n);
   v = P.alpha * v + bias;
   const int64_t off = m * P.ldc + n;
   if (P.preact) store_typed(P.preact, off, P.out_dtype, (P.act & kActStoreGrad) ? act_grad(v, P.act) : v);
@@ -94,6 +86,58 @@ __device__ __forceinline__ void split_finish(const SplitParams& P, float v, floa
   if (P.aux_mode) v = aux_apply(v, aux, P.aux_mode);
   if (P.accumulate) v += old;
   store_typed(P.C, off, P.out_dtype, v);
+}
+
+// One warp: the outputs (m0 + r, n0 + lane), r < 32, as chains of fp32 FMAs over the original operands; left in s[r * 33 + lane].
+// All of 8192 x 768 -> 3072: 0.63 ms with a NaN operand, which the first 32 k settle, 7.3 ms with an infinite one (CUDA-core kernel 1.4
+// ms; one lane per output inside the epilogue, as it was, kept the other roles in their bounded waits meanwhile).
+constexpr int kSpRedoPitch = 36;                     // rows of A: 16-byte reads
+constexpr int kSpRedo = 32 * (kSpRedoPitch + 33) * 4;        // its shared memory: 32 x 32 of A and of B
+static __device__ __noinline__ void split_redo(const SplitParams& P, int64_t m0, int64_t n0, float* s) {
+  const int lane = threadIdx.x & 31;
+  const float* A = (const float*)P.A;
+  const float* B = (const float*)P.B;
+  float* const as = s;                               // [row][k]
+  float* const bs = s + 32 * kSpRedoPitch;           // [k][column]
+  float acc[32];
+#pragma unroll
+  for (int r = 0; r < 32; ++r) acc[r] = 0.f;
+  for (int64_t k0 = 0; k0 < P.K; k0 += 32) {
+    __syncwarp();
+    for (int i0 = 0; i0 < 32; i0 += 8) {             // lanes walk the contiguous direction; zeros past the edges
+      float va[8], vb[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int64_t am = m0 + (P.trans_a ? lane : i0 + u), ak = k0 + (P.trans_a ? i0 + u : lane);
+        const int64_t bn = n0 + (P.trans_b ? i0 + u : lane), bk = k0 + (P.trans_b ? lane : i0 + u);
+        va[u] = am < P.M && ak < P.K ? A[P.trans_a ? ak * P.lda + am : am * P.lda + ak] : 0.f;
+        vb[u] = bn < P.N && bk < P.K ? B[P.trans_b ? bn * P.ldb + bk : bk * P.ldb + bn] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        as[P.trans_a ? lane * kSpRedoPitch + i0 + u : (i0 + u) * kSpRedoPitch + lane] = va[u];
+        bs[P.trans_b ? lane * 33 + i0 + u : (i0 + u) * 33 + lane] = vb[u];
+      }
+    }
+    __syncwarp();
+    // (the zeros behind the last k leave a sum as it is)
+    for (int k = 0; k < 32; k += 4) {
+      const float b0 = bs[k * 33 + lane], b1 = bs[(k + 1) * 33 + lane], b2 = bs[(k + 2) * 33 + lane], b3 = bs[(k + 3) * 33 + lane];
+#pragma unroll
+      for (int r = 0; r < 32; ++r) {
+        const float4 x = *reinterpret_cast<const float4*>(as + r * kSpRedoPitch + k);
+        acc[r] = fmaf(x.w, b3, fmaf(x.z, b2, fmaf(x.y, b1, fmaf(x.x, b0, acc[r]))));
+      }
+    }
+    bool done = true;                                // what is NaN stays NaN
+#pragma unroll
+    for (int r = 0; r < 32; ++r) done = done && (isnan(acc[r]) || m0 + r >= P.M);
+    if (__all_sync(0xffffffffu, done || n0 + lane >= P.N)) break;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 32; ++r) s[r * 33 + lane] = acc[r];
+  __syncwarp();
 }
 
 template <bool F32, bool A_MN, bool B_MN, bool PAIR>
@@ -115,6 +159,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * kSpSlots + 2 + b); };
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bar_ptr + 8 * (2 * kSpSlots + 4));
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* const redo_flag = abort_flag + 1;    // this CTA has outputs to make up
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int csize = PAIR ? 1 : P.csize;              // CTAs that split K
   const int prank = PAIR ? (int)cluster_ctarank() : 0;
@@ -125,6 +170,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int s = 0; s < kSpSlots; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), PAIR ? 2 * kSpEpiWarps : kSpEpiWarps); }
     *abort_flag = 0;
+    *redo_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -277,39 +323,48 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         for (int e = 0; e < NC; ++e) rows[e] = acc[e];
       } else {
         // thread = row becomes lane = column: rows of 128 bytes to and from global memory, any pitch
+        uint32_t left_out = 0;
 #pragma unroll
         for (int h = 0; h < NC / 32; ++h) {
           const int64_t n = n0 + h * 32 + lane;
           __syncwarp();
+          bool fine = true;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = acc[h * 32 + e];
+          for (int e = 0; e < 32; ++e) {
+            if (F32) fine = fine && split_finite(acc[h * 32 + e]);
+            stage[lane * 33 + e] = F32 ? acc[h * 32 + e] * kSpUnscale : acc[h * 32 + e];
+          }
+          if (F32 && __any_sync(0xffffffffu, !fine)) {
+            left_out |= 1u << h;
+            continue;
+          }
           __syncwarp();
           if (n < P.N) {
             const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
             const int rows = (int)min((int64_t)32, P.M - m0);
             const bool plain = !P.preact && !P.act && !P.aux_mode && !P.accumulate;
             for (int r0 = 0; r0 < rows; r0 += 8) {
-              float v[8];
-              bool fine = plain && r0 + 8 <= rows;
+              if (plain && r0 + 8 <= rows) {
+                float v[8];
 #pragma unroll
-              for (int u = 0; u < 8; ++u) {
-                v[u] = stage[(r0 + u) * 33 + lane];
-                fine = fine && (!F32 || fabsf(v[u]) <= 3.402823466e38f);
-              }
-              if (fine) {
+                for (int u = 0; u < 8; ++u) v[u] = stage[(r0 + u) * 33 + lane];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) store_typed(P.C, (m0 + r0 + u) * P.ldc + n, P.out_dtype, P.alpha * (F32 ? v[u] * kSpUnscale : v[u]) + bias);
+                for (int u = 0; u < 8; ++u) store_typed(P.C, (m0 + r0 + u) * P.ldc + n, P.out_dtype, P.alpha * v[u] + bias);
               } else {
-                // (kept small: eight copies of it in a row ran 15 % slower, on instruction fetches)
+                // (kept small: with eight copies of it in a row the kernel ran 15 % slower)
 #pragma unroll 2
                 for (int r = r0; r < min(r0 + 8, rows); ++r) {
                   const int64_t off = (m0 + r) * P.ldc + n;
-                  split_finish<F32>(P, stage[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
-                                    P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
+                  split_finish(P, stage[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
+                               P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
                 }
               }
             }
           }
+        }
+        if (F32 && lane == 0) {
+          P.left_out[((int64_t)t * (PAIR ? 2 : 1) + prank) * kSpEpiWarps + warp - 2] = (uint8_t)left_out;
+          if (left_out) *redo_flag = 1;
         }
       }
     }
@@ -319,12 +374,50 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (PAIR) cluster_sync_all();                        // neither CTA leaves, nor frees tensor memory, while its peer still works
+  // Makes the piece of 32 x 32 outputs at (m0, n0), rows of them, up; take(r, n) says which of its outputs are missing.
+  auto make_up = [&](int64_t m0, int64_t n0, int rows, float* scratch, auto&& take) {
+    split_redo(P, m0, n0, scratch);
+    const int64_t n = n0 + lane;
+    if (n < P.N) {
+      const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
+#pragma unroll 1
+      for (int r = 0; r < rows; ++r) {
+        if (!take(r, n)) continue;
+        const int64_t off = (m0 + r) * P.ldc + n;
+        split_finish(P, scratch[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
+                     P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
+      }
+    }
+    __syncwarp();
+  };
+  if (F32 && csize == 1 && *redo_flag && !*abort_flag) {
+    // the ring is idle: every copy into it was consumed by a product whose sum the epilogue has seen
+    float* const scratch = reinterpret_cast<float*>(base_ptr + warp * kSpRedo);
+    constexpr int kPieces = kSpEpiWarps * (NC / 32);
+    static_assert((kSpThreads / 32) * kSpRedo <= kSpSlots * kSpSlot, "scratch fits the ring");
+    for (int t = worker; t < total; t += workers) {
+      const int64_t mt0 = (int64_t)(P.n_fast ? t / P.tiles_n : t % P.tiles_m) * TM + prank * 128, nt0 = (int64_t)(P.n_fast ? t % P.tiles_n : t / P.tiles_m) * TN;
+      const uint8_t* marks = P.left_out + ((int64_t)t * (PAIR ? 2 : 1) + prank) * kSpEpiWarps;
+      for (int i = warp; i < kPieces; i += kSpThreads / 32) {
+        const int w = i / (NC / 32), h = i % (NC / 32);
+        const int64_t m0 = mt0 + ((w + 2) & 3) * 32, n0 = nt0 + (w >> 2) * NC + h * 32;
+        if ((marks[w] >> h & 1) && m0 < P.M && n0 < P.N) make_up(m0, n0, (int)min((int64_t)32, P.M - m0), scratch, [](int, int64_t) { return true; });
+      }
+    }
+  }
   if (!PAIR && csize > 1) {
     cluster_sync_all();
-    if (worker < total) {
-      const int64_t m0 = (int64_t)(P.n_fast ? worker / P.tiles_n : worker % P.tiles_m) * kSpM;
-      const int64_t n0 = (int64_t)(P.n_fast ? worker % P.tiles_n : worker / P.tiles_m) * kSpN;
-      const int share = kSpM / csize;
+    const bool have = worker < total;
+    const int64_t m0 = (int64_t)(P.n_fast ? worker / P.tiles_n : worker % P.tiles_m) * kSpM;
+    const int64_t n0 = (int64_t)(P.n_fast ? worker % P.tiles_n : worker / P.tiles_m) * kSpN;
+    const int share = kSpM / csize;
+    auto sum_at = [&](int r, int col, int c) { return mapa_shared(base + (uint32_t)(r * kSpPitch + col) * 4u, (uint32_t)c); };     // in CTA c
+    auto load_sum = [&](uint32_t at) {
+      float x;
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at) : "memory");
+      return x;
+    };
+    if (have) {
       float bias[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -340,18 +433,33 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (n < P.N && P.accumulate) old[j] = load_typed(P.C, off, P.out_dtype);
         }
         for (int c = 0; c < csize; ++c) {
-          const uint32_t src = mapa_shared(base + (uint32_t)(r * kSpPitch + lane) * 4u, (uint32_t)c);
+          const uint32_t at = sum_at(r, lane, c);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float x;
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(src + 128u * j) : "memory");
-            v[j] += x;
-          }
+          for (int j = 0; j < 4; ++j) v[j] += load_sum(at + 128u * j);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int64_t n = n0 + j * 32 + lane;
-          if (n < P.N) split_finish<F32>(P, v[j], bias[j], aux[j], old[j], m0 + r, n);
+          if (n >= P.N) continue;
+          if (F32 && !split_finite(v[j])) *redo_flag = 1;
+          else split_finish(P, F32 ? v[j] * kSpUnscale : v[j], bias[j], aux[j], old[j], m0 + r, n);
+        }
+      }
+    }
+    if (F32) {
+      __syncthreads();
+      if (have && *redo_flag && !*abort_flag) {        // the scratch lies behind the sums, which tell what is missing
+        float* const scratch = reinterpret_cast<float*>(base_ptr + (kSpM * kSpPitch * 4 + 127) / 128 * 128 + warp * kSpRedo);
+        static_assert((kSpM * kSpPitch * 4 + 127) / 128 * 128 + (kSpThreads / 32) * kSpRedo <= kSpSlots * kSpSlot, "sums and scratch fit the ring");
+        for (int i = warp; i < 4 * ((share + 31) / 32); i += kSpThreads / 32) {
+          const int r0 = rank * share + (i >> 2) * 32, col = (i & 3) * 32 + lane;
+          const int rows = (int)min((int64_t)min(32, (rank + 1) * share - r0), P.M - m0 - r0);
+          if (rows <= 0 || n0 + (i & 3) * 32 >= P.N) continue;
+          make_up(m0 + r0, n0 + (i & 3) * 32, rows, scratch, [&](int r, int64_t) {
+            float v = 0.f;
+            for (int c = 0; c < csize; ++c) v += load_sum(sum_at(r0 + r, col, c));
+            return !split_finite(v);
+          });
         }
       }
     }
@@ -426,7 +534,7 @@ constexpr double kSplitMinUs = 30.0;
 
 bool gemm_split_supported(const GemmArgs& g) {
   if (g.M < 16 || g.N < 16 || g.K < (g.in_dtype == MT_F32 ? 16 : 256)) return false;   // (half, K = 91: error 1.56e-7, FMA chain 1.46e-7)
-  if (g.M >= (1ll << 30) || g.N >= (1ll << 30) || g.K > (1ll << 17)) return false;   // (K: the time a row of plain dot products may take)
+  if (g.M >= (1ll << 30) || g.N >= (1ll << 30) || g.K > (1ll << 17)) return false;   // (K: as far as the error was measured)
   const double tiles = (double)((g.M + 63) / 64) * (double)((g.N + 63) / 64) / (0.87 * sm_count());
   return 8.0 + 0.05 * (double)g.K * (tiles > 1.0 ? tiles : 1.0) >= kSplitMinUs;
 }
@@ -479,6 +587,8 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
     at[i] = bytes;
     bytes += ((size_t)planes * rows[i] * j.pitch * 2 + 255) / 256 * 256;
   }
+  const size_t marks_at = bytes;
+  if (f32) bytes += 2 * (size_t)((g.M + 127) / 128) * (size_t)((g.N + 127) / 128) * kSpEpiWarps;      // (no fewer than a pair's tiles have)
   TempBuf tmp(bytes, st);
   if (!tmp.ok()) {                                                   // no room for the planes
     cudaGetLastError();
@@ -514,6 +624,7 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
   // Slices that stay in tensor memory: the error grows with them, the FMA chain's with sqrt(K), and the epilogue's additions
   // cost time (3885 x 50257 -> 768: one slice 700 us, two 585, four 515, eight 479).
   P.chunk = f32 || g.K < 2048 ? 1 : g.K < 12288 ? 2 : g.K < 49152 ? 4 : 8;
+  P.left_out = f32 ? (uint8_t*)tmp.ptr + marks_at : nullptr;
   P.flag = device_flag_ptr();
   // Neighbouring tiles share the larger operand's panel unless it fits the L2 anyway.
   P.n_fast = g.M > g.N ? 1 : 0;

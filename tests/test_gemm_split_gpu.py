@@ -151,3 +151,43 @@ def test_values_that_are_not_finite_come_out_as_in_fp32(mt, M, N, K):
     rows = np.isfinite(a).all(1)
     exact, size = product(a[rows], b, 0, 1)
     assert (np.abs(got[rows] - exact) <= bound(K) * size)[np.isfinite(want[rows])].all()
+
+
+# many pieces to make up: whole operands, single rows and columns, results above the planes' range; one CTA, a pair and a
+# cluster per tile, several tiles per CTA, every operand order, and the outputs that read what was there
+@pytest.mark.parametrize("ta,tb", ORDERS)
+@pytest.mark.parametrize("M,N,K", [(300, 260, 500), (130, 70, 2000), (2600, 2500, 130), (40, 300, 4096)])
+@pytest.mark.parametrize("where", ["all", "row", "column", "large"])
+def test_pieces_left_out_are_made_up(mt, M, N, K, ta, tb, where):
+    F = mt.fused_ops
+    r = np.random.default_rng(7)
+    a, b = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    if where == "all":
+        a[:] = np.nan
+    elif where == "row":
+        a[M // 2, K - 1] = np.inf
+    elif where == "column":
+        b[N - 1, 0] = np.nan
+    else:
+        a[M // 3], b[N // 2] = a[M // 3] * np.float32(1e20), b[N // 2] * np.float32(1e15)
+    A, B = dev(mt, np.ascontiguousarray(a.T) if ta else a, "float32"), dev(mt, b if tb else np.ascontiguousarray(b.T), "float32")
+    aux, bias = dev(mt, r.standard_normal((M, N)).astype(np.float32), "float32"), dev(mt, r.standard_normal(N).astype(np.float32), "float32")
+
+    def outputs():
+        c = dev(mt, aux.numpy(), "float32")
+        y, pre = F.gemm(A, B, trans_a=bool(ta), trans_b=bool(tb), bias=bias, act="gelu", preact=True)
+        return [F.gemm(A, B, trans_a=bool(ta), trans_b=bool(tb)).numpy(), F.gemm(A, B, trans_a=bool(ta), trans_b=bool(tb), out=c, accumulate=1).numpy(),
+                F.gemm(A, B, trans_a=bool(ta), trans_b=bool(tb), aux=aux, aux_mode=1).numpy(), y.numpy(), pre.numpy()]
+    got = outputs()
+    mt._lib.gemm_force_simt(1)
+    try:
+        want = outputs()
+    finally:
+        mt._lib.gemm_force_simt(0)
+    size = np.abs(np.nan_to_num(a, posinf=0)).astype(np.float64) @ np.abs(np.nan_to_num(b)).T.astype(np.float64)
+    for i, (g, w) in enumerate(zip(got, want)):
+        assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(np.isinf(g), np.isinf(w)), i
+        ok = np.isfinite(w)
+        # both sides' sums; bias, aux and old values of size one; GELU's slope of up to 1.13
+        assert (np.abs(g.astype(np.float64) - w) <= (bound(K) + (K + 4) * 2.0 ** -24) * 1.2 * (size + 8))[ok].all(), i
+    no_device_flag(mt)
