@@ -81,3 +81,34 @@ def test_strided_rows_in_one_buffer(mt, offset, row):
                   D ** -0.5, 1, X.code, stream())
     for g, w, name in zip([O, L] + grads, want, ("o", "lse", "dq", "dk", "dv")):
         close(g.numpy(), w, 2e-5, name)
+
+
+# a row in the first, a middle and the last of the 64-row tiles; both block heights, grouped heads, every padded head size
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("dtype,B,H,Hk,S,D,t", [("float32", 1, 2, 1, 200, 64, 70), ("float32", 7, 16, 16, 260, 64, 127), ("float32", 1, 2, 2, 130, 32, 63),
+                                                ("float32", 7, 16, 8, 257, 128, 200), ("float32", 1, 4, 4, 129, 90, 128), ("float16", 1, 2, 2, 140, 96, 3)])
+def test_masked_values_that_are_not_finite_reach_no_row(mt, dtype, B, H, Hk, S, D, t, bad):
+    """Row t of one operand is not finite: causal attention gives the rows that do not see it what it gives without it."""
+    F = mt.fused_ops
+    r = np.random.default_rng(S + D)
+    clean = [rnd(r.standard_normal((B, h, S, D)), dtype) for h in (H, Hk, Hk, H)]
+    want = reference(*clean, True)
+    tol = 2e-5 if dtype == "float32" else TOL[dtype]
+
+    def run(which):
+        arrays = [a.copy() for a in clean]
+        if which is not None:
+            arrays[which][:, :, t, ::3] = bad
+        Q, K, V, G = (dev(mt, a, dtype) for a in arrays)
+        Q, K, V, o, lse = F.fused_sdpa_forward(Q, K, V, causal=True)
+        return [a.numpy() for a in (o, lse) + tuple(F.fused_sdpa_backward(G, Q, K, V, o, lse, causal=True))]
+    before, after = slice(0, t), slice(t + 1, S)
+    # operand -> what does not depend on its row t: rows of o, lse and dq before a key's, of dk and dv behind a query's
+    for which, parts in ((0, {0: before, 1: before, 2: before, 3: after, 4: after}), (1, {0: before, 1: before, 2: before}),
+                         (2, {0: before, 2: before}), (3, {2: before, 3: after, 4: after})):
+        got = run(which)
+        for i, rows in parts.items():
+            if rows.start < rows.stop:
+                close(got[i][:, :, rows], want[i][:, :, rows], tol, f"operand {which}, result {i}")
+        if which == 2:
+            assert not np.isfinite(got[0][:, :, t, ::3]).any()
