@@ -170,7 +170,13 @@ attn_decode_kernel(const DecodeParams p) {
         s[u] = j0 + u * KPI + grp < j_end ? dot : -INFINITY;
         mx = fmaxf(mx, s[u]);
       }
-      if (mx == -INFINITY) continue;       // no key of this lane group yet (per lane; no shuffles below)
+      if (mx == -INFINITY) {               // no key of this lane group yet (per lane; no shuffles below), or only NaN scores
+        bool nan = false;
+#pragma unroll
+        for (int u = 0; u < U; ++u) nan |= isnan(s[u]);
+        if (!nan) continue;
+        mx = 0.f;
+      }
       const float alpha = exp2f(m[g] - mx);
       m[g] = mx;
       l[g] *= alpha;
@@ -220,7 +226,7 @@ attn_decode_kernel(const DecodeParams p) {
       ll += red_l[w][g] * a;
       v += red_o[w][g][d] * a;
     }
-    if (splits == 1) out(g, d, ll > 0.f ? v / ll : 0.f);
+    if (splits == 1) out(g, d, ll == 0.f ? 0.f : v / ll);
     else {
       part_o[g][d] = v;
       if (d == 0) { part_m[g] = mm; part_l[g] = ll; }
@@ -238,7 +244,7 @@ attn_decode_kernel(const DecodeParams p) {
         ll += *cluster.map_shared_rank(&part_l[g], r) * a;
         v += *cluster.map_shared_rank(&part_o[g][d], r) * a;
       }
-      out(g, d, ll > 0.f ? v / ll : 0.f);
+      out(g, d, ll == 0.f ? 0.f : v / ll);
     }
     cluster.sync();                        // nobody leaves while its partial is still being read
   }
