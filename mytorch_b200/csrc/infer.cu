@@ -91,11 +91,15 @@ int Infer::run() {
   const size_t bx = up256((size_t)M * E * es), bqkv = up256((size_t)M * nqkv * es), bmlp = up256((size_t)M * F * es);
   const size_t brope = learned || step ? 0 : up256((size_t)M * (nq + nkv) * es);
   const size_t blse = step ? 0 : up256((size_t)M * H * 4), brstd = learned || step ? 0 : 2 * blse;
-  TempBuf buf(3 * bx + bqkv + bmlp + brope + blse + brstd, st);
+  // Two regions serve twice per block, so that what a kernel reads is still in the L2: the normed rows are dead when attention
+  // writes its output, the projections when the up-projection writes the hidden rows.
+  const size_t bwide = bqkv + brope > bmlp ? bqkv + brope : bmlp;
+  TempBuf buf(2 * bx + bwide + blse + brstd, st);
   if (!buf.ok()) return MT_ERR_CUDA;
   char* at = (char*)buf.ptr;
   auto take = [&](size_t n) { char* p = at; at += n; return p; };
-  char *x = take(bx), *h = take(bx), *att = take(bx), *qkv = take(bqkv), *mlp = take(bmlp), *roped = take(brope);
+  char *x = take(bx), *h = take(bx), *qkv = take(bwide);
+  char *att = h, *mlp = qkv, *roped = qkv + bqkv;
   float* lse = (float*)take(blse);
   float* rstd = (float*)take(brstd);
   void* stream = (void*)st;
@@ -150,8 +154,8 @@ int Infer::run() {
   int64_t rows = M;
   const void* last = x;
   if (s.last_only && T > 1) {                // the head only sees each sequence's last position
-    MT_CHECK_CUDA(cudaMemcpy2DAsync(att, E * es, x + (T - 1) * E * es, T * E * es, E * es, B, cudaMemcpyDeviceToDevice, st));
-    last = att;
+    MT_CHECK_CUDA(cudaMemcpy2DAsync(qkv, E * es, x + (T - 1) * E * es, T * E * es, E * es, B, cudaMemcpyDeviceToDevice, st));
+    last = qkv;
     rows = B;
   }
   const int64_t nv[1] = {g.vocab};
