@@ -50,5 +50,6 @@ bool gemm_split_supported(const GemmArgs& g);      // fp32, and half operands th
 int gemm_split(const GemmArgs& g, cudaStream_t st);
 bool gemm_tc_supported(const GemmArgs& g);
 int gemm_tc(const GemmArgs& g, cudaStream_t st);
+bool gemm_automatic();         // neither mt_gemm_force_simt nor mt_gemm_tile_policy is set
 int resident_cta_pairs();      // clusters of two CTAs that take an SM each and run at the same time
 }  // namespace mt

@@ -951,6 +951,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t st) {
 using namespace mt;
 
 static int g_force_simt = 0;
+bool mt::gemm_automatic() { return !g_force_simt && g_tile_policy == 0; }
 
 extern "C" {
 
@@ -990,7 +991,7 @@ int mt_gemm_ex(const void* A, const void* B, void* C, void* preact, const void* 
   g.aux = aux;
   g.aux_mode = aux_mode;
   cudaStream_t st = as_stream(stream);
-  if (!g_force_simt && g_tile_policy == 0 && M <= kSkinnyMaxRows && !trans_a && trans_b && !accumulate && !preact && alpha == 1.f &&
+  if (gemm_automatic() && M <= kSkinnyMaxRows && !trans_a && trans_b && !accumulate && !preact && alpha == 1.f &&
       aux_mode <= 1 && in_dtype == out_dtype) {
     SkinnyArgs a;
     a.x = A; a.ldx = lda; a.M = (int)M; a.K = (int)K; a.dtype = in_dtype;

@@ -44,7 +44,7 @@ struct Infer {
     a.norm = norm_kind(); a.gamma = nw; a.beta = nb; a.eps = g.eps;
     a.early_weights = 1;
     SkinnyShape shape;
-    if (rows <= kFusedNormRows && skinny_fits(a, shape)) return skinny_gemm(a, shape, st);
+    if (gemm_automatic() && rows <= kFusedNormRows && skinny_fits(a, shape)) return skinny_gemm(a, shape, st);
     int rc = norm(x, nw, nb, h, rows);
     int64_t col = 0;
     for (int i = 0; i < nseg && !rc; ++i) {
@@ -62,7 +62,7 @@ struct Infer {
     a.w[0] = w; a.bias[0] = bias; a.n[0] = (int)E; a.ldw = K;
     a.out = x; a.ldo = E; a.residual = x; a.early_weights = 1;
     SkinnyShape shape;
-    if (skinny_fits(a, shape)) return skinny_gemm(a, shape, st);
+    if (gemm_automatic() && skinny_fits(a, shape)) return skinny_gemm(a, shape, st);
     return mt_gemm_ex(a_, w, x, nullptr, bias, x, 1, rows, E, K, K, K, E, 0, 1, g.dtype, g.dtype, 0, 1.f, 0, (void*)st);
   }
   mt_strides3 rows_of(int64_t ld, int64_t d) const { return mt_strides3{s.new_tokens * ld, d, ld}; }

@@ -126,6 +126,21 @@ def test_wide_norm_and_head(mt, monkeypatch, dtype, width, B):
     no_device_flag(mt)
 
 
+def test_forced_kernels_are_used(mt, monkeypatch):
+    """mt_gemm_force_simt holds for the products inside the library call: bit for bit the layers' results."""
+    from mytorch_b200 import infer
+    model = models(mt, "gpt2", "float32", 2, 2, 64, True)
+    x = mt.Tensor(np.arange(5, dtype=np.int32)[None])
+    mt._lib.gemm_force_simt(1)
+    try:
+        with mt.no_grad():
+            one_call = model(x).numpy()
+            monkeypatch.setattr(infer, "plan_of", lambda m, b: None)
+            assert np.array_equal(one_call, model(x).numpy())
+    finally:
+        mt._lib.gemm_force_simt(0)
+
+
 def test_plans_follow_the_weights(mt):
     """Replaced, cast or reloaded weights are used by the next forward."""
     model = models(mt, "gpt2", "float32", 2, 2, 64, False)
