@@ -1,5 +1,9 @@
 """The whole-model forward (mt_gpt_forward), the few-row products under it and the device arg-max,
 against the op-by-op path of the same models and NumPy."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -139,6 +143,53 @@ def test_forced_kernels_are_used(mt, monkeypatch):
             assert np.array_equal(one_call, model(x).numpy())
     finally:
         mt._lib.gemm_force_simt(0)
+
+
+# K up to the longest that goes there, split over a cluster of eight
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K", [(1, 72, 32768), (9, 100, 12288), (33, 40, 8192)])
+def test_few_rows_of_long_k(mt, dtype, M, N, K):
+    r = np.random.default_rng(K)
+    a, w = rnd(r.standard_normal((M, K)), dtype), rnd(r.standard_normal((N, K)) / np.sqrt(K), dtype)
+    got = mt.fused_ops.gemm(dev(mt, a, dtype), dev(mt, w, dtype), trans_b=True).numpy()
+    close(got, a.astype(np.float64) @ w.T.astype(np.float64), TOL[dtype])
+    no_device_flag(mt)
+
+
+def steps(mt, kind):
+    """Logits of a prompt and of steps behind it: the five-kernel schedule."""
+    model = models(mt, kind, "float16", 4, 2, 64, True)
+    ids = np.random.default_rng(5).integers(0, 200, (3, 70)).astype(np.int32)
+    cache, got = cache_of(mt, model, kind, 3), []
+    with mt.no_grad():
+        for p in [ids[:, :64]] + [ids[:, t:t + 1] for t in range(64, 70)]:
+            out = model(mt.Tensor(p), cache=cache) if kind == "gpt2" else model(mt.Tensor(p), None, cache=cache)
+            got.append(out[0].numpy()[:, -1])
+    return np.stack(got)
+
+
+@pytest.mark.parametrize("kind", ["gpt2", "nanochat"])
+def test_steps_without_overlap_and_on_another_stream(mt, tmp_path, kind):
+    """Kernels that start before their predecessor has ended read nothing that it writes: the same bits with the overlap
+    off (MT_PDL=0, read once per process), and on a stream of the caller's."""
+    import ctypes as C
+    from mytorch_b200 import _lib, array
+    want = steps(mt, kind)
+    code = f"import mytorch_b200 as mt, numpy as np, tests.test_infer_gpu as t; np.save({str(tmp_path / 'x.npy')!r}, t.steps(mt, {kind!r}))"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    child = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, MT_PDL="0"), capture_output=True, text=True, timeout=300)
+    assert child.returncode == 0, child.stderr[-2000:]
+    assert np.array_equal(np.load(tmp_path / "x.npy"), want)
+    mine, before = C.c_void_p(), array.stream()
+    array.synchronize()
+    _lib.stream_create(C.byref(mine))
+    array.set_stream(mine)
+    try:
+        assert np.array_equal(steps(mt, kind), want)
+        array.synchronize()
+    finally:
+        array.set_stream(before)
+    _lib.stream_destroy(mine)
 
 
 def test_plans_follow_the_weights(mt):
