@@ -88,35 +88,37 @@ __device__ __forceinline__ void split_finish(const SplitParams& P, float v, floa
   store_typed(P.C, off, P.out_dtype, v);
 }
 
-// One warp: the outputs (m0 + r, n0 + lane), r < 32, as chains of fp32 FMAs over the original operands; left in s[r * 33 + lane].
-// All of 8192 x 768 -> 3072: 0.63 ms with a NaN operand, which the first 32 k settle, 7.3 ms with an infinite one (CUDA-core kernel 1.4
-// ms; one lane per output inside the epilogue, as it was, kept the other roles in their bounded waits meanwhile).
+// One warp: the outputs (m0 + r, n0 + lane) whose bit r is set in the lane's `missing`, as chains of fp32 FMAs over the original operands.
+// Its own function, and the parameters stay where they are (__grid_constant__): inlined, it cost the kernel 2-4 us. All of
+// 8192 x 768 -> 3072: 0.66 ms with a NaN operand, which the first 32 k settle, 4.6 ms with an infinite one (the CUDA-core kernel 1.4).
 constexpr int kSpRedoPitch = 36;                     // rows of A: 16-byte reads
 constexpr int kSpRedo = 32 * (kSpRedoPitch + 33) * 4;        // its shared memory: 32 x 32 of A and of B
-static __device__ __noinline__ void split_redo(const SplitParams& P, int64_t m0, int64_t n0, float* s) {
+static __device__ __noinline__ void split_make_up(const SplitParams& P, int64_t m0, int64_t n0, uint32_t missing, float* s) {
   const int lane = threadIdx.x & 31;
   const float* A = (const float*)P.A;
   const float* B = (const float*)P.B;
+  const int64_t M = P.M, N = P.N, K = P.K, lda = P.lda, ldb = P.ldb;
+  const bool ta = P.trans_a, tb = P.trans_b;
   float* const as = s;                               // [row][k]
   float* const bs = s + 32 * kSpRedoPitch;           // [k][column]
   float acc[32];
 #pragma unroll
   for (int r = 0; r < 32; ++r) acc[r] = 0.f;
-  for (int64_t k0 = 0; k0 < P.K; k0 += 32) {
+  for (int64_t k0 = 0; k0 < K; k0 += 32) {
     __syncwarp();
     for (int i0 = 0; i0 < 32; i0 += 8) {             // lanes walk the contiguous direction; zeros past the edges
       float va[8], vb[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const int64_t am = m0 + (P.trans_a ? lane : i0 + u), ak = k0 + (P.trans_a ? i0 + u : lane);
-        const int64_t bn = n0 + (P.trans_b ? i0 + u : lane), bk = k0 + (P.trans_b ? lane : i0 + u);
-        va[u] = am < P.M && ak < P.K ? A[P.trans_a ? ak * P.lda + am : am * P.lda + ak] : 0.f;
-        vb[u] = bn < P.N && bk < P.K ? B[P.trans_b ? bn * P.ldb + bk : bk * P.ldb + bn] : 0.f;
+        const int64_t am = m0 + (ta ? lane : i0 + u), ak = k0 + (ta ? i0 + u : lane);
+        const int64_t bn = n0 + (tb ? i0 + u : lane), bk = k0 + (tb ? lane : i0 + u);
+        va[u] = am < M && ak < K ? A[ta ? ak * lda + am : am * lda + ak] : 0.f;
+        vb[u] = bn < N && bk < K ? B[tb ? bn * ldb + bk : bk * ldb + bn] : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        as[P.trans_a ? lane * kSpRedoPitch + i0 + u : (i0 + u) * kSpRedoPitch + lane] = va[u];
-        bs[P.trans_b ? lane * 33 + i0 + u : (i0 + u) * 33 + lane] = vb[u];
+        as[ta ? lane * kSpRedoPitch + i0 + u : (i0 + u) * kSpRedoPitch + lane] = va[u];
+        bs[tb ? lane * 33 + i0 + u : (i0 + u) * 33 + lane] = vb[u];
       }
     }
     __syncwarp();
@@ -131,18 +133,30 @@ static __device__ __noinline__ void split_redo(const SplitParams& P, int64_t m0,
     }
     bool done = true;                                // what is NaN stays NaN
 #pragma unroll
-    for (int r = 0; r < 32; ++r) done = done && (isnan(acc[r]) || m0 + r >= P.M);
-    if (__all_sync(0xffffffffu, done || n0 + lane >= P.N)) break;
+    for (int r = 0; r < 32; ++r) done = done && (isnan(acc[r]) || m0 + r >= M);
+    if (__all_sync(0xffffffffu, done || n0 + lane >= N)) break;
   }
   __syncwarp();
 #pragma unroll
   for (int r = 0; r < 32; ++r) s[r * 33 + lane] = acc[r];
   __syncwarp();
+  const int64_t n = n0 + lane;
+  if (n < P.N) {
+    const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
+#pragma unroll 1
+    for (int r = 0; r < 32; ++r) {
+      if (!(missing >> r & 1)) continue;
+      const int64_t off = (m0 + r) * P.ldc + n;
+      split_finish(P, s[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
+                   P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
+    }
+  }
+  __syncwarp();
 }
 
 template <bool F32, bool A_MN, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(kSpThreads, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitParams P) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ SplitParams P) {
   constexpr int PLANES = F32 ? 3 : 1;
   constexpr int TM = PAIR ? 256 : 128, TN = PAIR ? 256 : 128;      // tile of a CTA or a pair; either way a CTA stages 128 rows of A and of B
   constexpr int NC = TN / 2;                         // columns an epilogue warp holds
@@ -374,22 +388,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (PAIR) cluster_sync_all();                        // neither CTA leaves, nor frees tensor memory, while its peer still works
-  // Makes the piece of 32 x 32 outputs at (m0, n0), rows of them, up; take(r, n) says which of its outputs are missing.
-  auto make_up = [&](int64_t m0, int64_t n0, int rows, float* scratch, auto&& take) {
-    split_redo(P, m0, n0, scratch);
-    const int64_t n = n0 + lane;
-    if (n < P.N) {
-      const float bias = P.bias ? load_typed(P.bias, n, P.in_dtype) : 0.f;
-#pragma unroll 1
-      for (int r = 0; r < rows; ++r) {
-        if (!take(r, n)) continue;
-        const int64_t off = (m0 + r) * P.ldc + n;
-        split_finish(P, scratch[r * 33 + lane], bias, P.aux_mode ? load_typed(P.aux, off, P.out_dtype) : 0.f,
-                     P.accumulate ? load_typed(P.C, off, P.out_dtype) : 0.f, m0 + r, n);
-      }
-    }
-    __syncwarp();
-  };
+  auto rows_mask = [](int rows) { return 0xffffffffu >> (32 - rows); };
   if (F32 && csize == 1 && *redo_flag && !*abort_flag) {
     // the ring is idle: every copy into it was consumed by a product whose sum the epilogue has seen
     float* const scratch = reinterpret_cast<float*>(base_ptr + warp * kSpRedo);
@@ -401,7 +400,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       for (int i = warp; i < kPieces; i += kSpThreads / 32) {
         const int w = i / (NC / 32), h = i % (NC / 32);
         const int64_t m0 = mt0 + ((w + 2) & 3) * 32, n0 = nt0 + (w >> 2) * NC + h * 32;
-        if ((marks[w] >> h & 1) && m0 < P.M && n0 < P.N) make_up(m0, n0, (int)min((int64_t)32, P.M - m0), scratch, [](int, int64_t) { return true; });
+        if ((marks[w] >> h & 1) && m0 < P.M && n0 < P.N) split_make_up(P, m0, n0, rows_mask((int)min((int64_t)32, P.M - m0)), scratch);
       }
     }
   }
@@ -455,11 +454,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const int r0 = rank * share + (i >> 2) * 32, col = (i & 3) * 32 + lane;
           const int rows = (int)min((int64_t)min(32, (rank + 1) * share - r0), P.M - m0 - r0);
           if (rows <= 0 || n0 + (i & 3) * 32 >= P.N) continue;
-          make_up(m0 + r0, n0 + (i & 3) * 32, rows, scratch, [&](int r, int64_t) {
+          uint32_t missing = 0;
+          for (int r = 0; r < rows; ++r) {
             float v = 0.f;
             for (int c = 0; c < csize; ++c) v += load_sum(sum_at(r0 + r, col, c));
-            return !split_finite(v);
-          });
+            if (!split_finite(v)) missing |= 1u << r;
+          }
+          if (__any_sync(0xffffffffu, missing)) split_make_up(P, m0 + r0, n0 + (i & 3) * 32, missing, scratch);
         }
       }
     }
