@@ -271,8 +271,11 @@ int mt_rope_rmsnorm_bwd(const void* dyq, const void* dyk, const void* yq, const 
  * op(B) is [K,N]: trans_b=0 -> B stored [K,N] (ldb>=N); trans_b=1 -> B stored [N,K].
  * Linear forward is (trans_a=0, trans_b=1); dgrad (0,0); wgrad (1,0).
  * in_dtype f16/bf16 runs on tcgen05 tensor cores (fp32 accumulate in TMEM)
- * when pointers/strides are 16-byte aligned, else on a CUDA-core kernel;
- * in_dtype f32 runs on the CUDA-core kernel in full fp32.
+ * when pointers/strides are 16-byte aligned. Other half products with K >= 256
+ * and f32 products run there too once they are large (copied with a 16-byte
+ * pitch; f32 as three bf16 planes per operand), with sums no further from 64
+ * bits than a chain of fp32 FMAs; small ones run on a CUDA-core kernel. Up to
+ * 64 rows times a transposed B stream B instead.
  * bias: [N] in in_dtype or NULL. preact: optional second output receiving the
  * value before the activation (same dtype/ld as C), or NULL.
  * accumulate: 0 = overwrite, 1 = C += result (read-modify-write),

@@ -1,5 +1,5 @@
 // CUDA-core GEMM with fp32 accumulation: small products in fp32 or with pointers
-// or pitches that TMA cannot address (gemm_split.cu takes the larger ones), and
+// or pitches that TMA cannot address (gemm_split.cu takes the larger ones; half types below K = 256), and
 // the independent check of the tensor-core kernels. 64x64x16 tiles,
 // 256 threads, 4x4 outputs per thread, any strides / transposes / tails.
 #include "common.cuh"

@@ -17,12 +17,13 @@
 //
 // Persistent. A slot of a CTA's ring holds 128 rows of one plane of A and of B (2 x 16 KB), a 64-deep slice of fp32
 // operands three slots. A CTA pair (cta_group::2) works on a 256 x 256 tile: the 24 MMAs of a slice last 3072 tensor
-// cycles while the ring's other half fills. A single CTA's 128 x 128 tile lasts 1536 and waits for its 96 KB (64 B per clock
-// and SM, and as long a way from L2 as the MMAs take); it is there for products with too few tiles. Where even those are few
+// cycles while the ring's other half fills. A single CTA's 128 x 128 tile has 1536 cycles of MMAs for the same 96 KB
+// and measures 3600 a slice; it is there for products with too few tiles. Where even those are few
 // (weight gradients of small layers), K is split over a cluster of up to eight CTAs whose sums meet
 // through distributed shared memory in a fixed order: no atomics, the same bits every time.
-// fp32: 8192 x 768 -> 3072 1414 -> 202 us, its weight gradient 1529 -> 260, 4096 x 256 -> 1024 102 -> 25, 256 x 4096 x 256
-// 209 -> 25; bf16 with odd pitches and fp32 output: 50257 x 3885 -> 768 12345 -> 526 us.
+// Against the CUDA-core kernel, fp32: 8192 x 768 -> 3072 1417 -> 179 us (tensor pipe 60 % of its cycles; with GELU and the second
+// output 27 %, for the next tile's MMAs do not hide that epilogue), its weight gradient 1547 -> 242, 4096 x 256 -> 1024 106 -> 21,
+// 256 x 4096 x 256 212 -> 26; bf16 with odd pitches: 50257 x 3885 -> 768 to fp32 12390 -> 464 us, 3885 x 50257 -> 768 15420 -> 457.
 //
 // A sum that is not finite (an operand is, or one is above 2^103, or the result above 2^79) is computed again as a plain
 // chain of fp32 FMAs, so infinities and NaNs come out as fp32 arithmetic gives them. The epilogue only leaves such 32 x 32
@@ -642,7 +643,7 @@ int gemm_split(const GemmArgs& g, cudaStream_t st) {
   }
   // A pair's 256 x 256 tile needs half the operand bytes per multiplication: a slice takes it about 4300
   // cycles, a single CTA's 128 x 128 tile 3600 (one plane: 1990, 1770); which one is ahead is a matter of how many rounds
-  // of tiles each leaves on the chip (fp32 8192 x 768 -> 3072: pair 202 us, single 423; 3072 x 8192 x 768: 308, 260).
+  // of tiles each leaves on the chip (fp32 8192 x 768 -> 3072: pair 179 us, single 423; 3072 x 8192 x 768: 308, 260).
   const double kb_one = f32 ? 3600.0 : 1770.0, kb_pair = f32 ? 4300.0 : 1990.0;
   const double one = (double)((tiles * P.csize + sms - 1) / sms) * (P.kb_per_rank * kb_one + 4000.0);
   const double two = (double)((tiles_of(256) + pairs - 1) / pairs) * (P.kb_total * kb_pair + 6000.0);

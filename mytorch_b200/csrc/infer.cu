@@ -1,6 +1,7 @@
 // Forward pass of a whole GPT model without a graph (scoring, prompts, decoding steps): one library
 // call queues every kernel of the model. Called op by op from Python a decoding step of a 12-block
-// model is about 100 calls and 1.9 ms of host time around 0.15 ms of GPU work.
+// model is about 100 calls and 1.9 ms of host time around 0.37 ms on the device (124 M parameters, fp16, 8 sequences; queueing
+// its 62 launches from here takes 0.35 ms).
 //
 // Two schedules. A step with one new token per sequence (and few sequences) runs five kernels per
 // block: {norm + q/k/v}, {rotary + QK-norm + cache append + attention}, {output projection +
