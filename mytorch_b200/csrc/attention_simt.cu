@@ -41,12 +41,9 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
   return r;
 }
 
-// dst[r][d] = mul * src row row0 + r, r < ROWS, d < DP: zero past the sequence and past D. With `look` it says whether
-// this thread saw a value that is not finite.
+// dst[r][d] = mul * src row row0 + r, r < ROWS, d < DP: zero past the sequence and past D.
 template <typename T, int DP, int ROWS>
-__device__ __forceinline__ bool load_rows(float* dst, const T* src, int64_t stride, int row0, int total, int D, float mul, bool vec,
-                                          bool look = false) {
-  bool odd = false;
+__device__ __forceinline__ void load_rows(float* dst, const T* src, int64_t stride, int row0, int total, int D, float mul, bool vec) {
   constexpr int VN = Vec16<T>::N, PER = DP / VN;
   if (vec) {
 #pragma unroll 4
@@ -59,17 +56,23 @@ __device__ __forceinline__ bool load_rows(float* dst, const T* src, int64_t stri
       for (int e = 0; e < VN; e += 4)
         *reinterpret_cast<float4*>(dst + r * (DP + 4) + c + e) =
             make_float4(t.get(e) * mul, t.get(e + 1) * mul, t.get(e + 2) * mul, t.get(e + 3) * mul);
-      if (look)
-#pragma unroll
-        for (int e = 0; e < VN; ++e) odd |= !isfinite(t.get(e));
     }
   } else {
     for (int i = threadIdx.x; i < ROWS * DP; i += kAtThreads) {
       const int r = i / DP, c = i - r * DP;
-      const float v = row0 + r < total && c < D ? to_f(src[(int64_t)(row0 + r) * stride + c]) : 0.f;
-      dst[r * (DP + 4) + c] = v * mul;
-      odd |= !isfinite(v);
+      dst[r * (DP + 4) + c] = row0 + r < total && c < D ? to_f(src[(int64_t)(row0 + r) * stride + c]) * mul : 0.f;
     }
+  }
+}
+
+// Whether this thread's part of a 64-row tile in shared memory holds a value that is not finite.
+template <int DP>
+__device__ __forceinline__ bool tile_odd(const float* tile) {
+  bool odd = false;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < kAtCols * DP / 4; i += kAtThreads) {
+    const float4 v = *reinterpret_cast<const float4*>(tile + i / (DP / 4) * (DP + 4) + i % (DP / 4) * 4);
+    odd |= !(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w));
   }
   return odd;
 }
@@ -122,14 +125,14 @@ __device__ __forceinline__ void combine(uint64_t (&acc)[TI][DP / 32], const floa
   }
 }
 
-// The same over row i's j in [lo[i], hi[i]) alone: whatever stands in the other rows of x is not touched.
+// The same over row i's j in [lo + 2 i, hi + 2 i) alone: whatever stands in the other rows of x, or for them in w, is not touched.
 template <int DP, int TI>
-__device__ __forceinline__ void combine_visible(uint64_t (&acc)[TI][DP / 32], const float* w, const float* x, const int (&lo)[TI], const int (&hi)[TI]) {
+__device__ __forceinline__ void combine_visible(uint64_t (&acc)[TI][DP / 32], const float* w, const float* x, int lo, int hi) {
 #pragma unroll 1
   for (int j = 0; j < kAtCols; ++j) {
 #pragma unroll
     for (int i = 0; i < TI; ++i) {
-      if (j < lo[i] || j >= hi[i]) continue;
+      if (j < lo + 2 * i || j >= hi + 2 * i) continue;
       const float q = w[i * 2 * kAtPitch + j];
       const uint64_t q2 = pack2(q, q);
 #pragma unroll
@@ -192,9 +195,11 @@ attn_fwd_simt(const SimtParams P) {
   const int kv_end = P.causal ? min(row_base + ROWS, S) : S;
   for (int t0 = 0; t0 < kv_end; t0 += kAtCols) {
     __syncthreads();
-    const bool diagonal = P.causal && t0 + kAtCols > row_base + 1;        // some row does not see all of it
     load_rows<T, DP, kAtCols>(Ks, kb, P.sk.s, t0, S, D, 1.f, P.vec);
-    const int odd = __syncthreads_or(load_rows<T, DP, kAtCols>(Vs, vb, P.sv.s, t0, S, D, 1.f, P.vec, diagonal));
+    load_rows<T, DP, kAtCols>(Vs, vb, P.sv.s, t0, S, D, 1.f, P.vec);
+    __syncthreads();
+    bool odd = false;                                       // on the diagonal: rows that not every query sees, and not all finite
+    if (P.causal && t0 + kAtCols > row_base + 1) odd = __syncthreads_or(tile_odd<DP>(Vs));
     if (P.causal && t0 > warp_last) continue;               // no row of this warp sees the tile
     float s[TI][4];
     dots<DP, TI>(s, Qs + r0 * (DP + 4), Ks + tx * (DP + 4));
@@ -231,14 +236,8 @@ attn_fwd_simt(const SimtParams P) {
       for (int p = 0; p < DP / 32; ++p) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][p]) : "l"(c2));
     }
     __syncwarp();
-    if (diagonal && odd) {
-      int lo[TI], hi[TI];
-#pragma unroll
-      for (int i = 0; i < TI; ++i) { lo[i] = 0; hi[i] = row_base + r0 + 2 * i + 1 - t0; }
-      combine_visible<DP, TI>(acc, Ps + r0 * kAtPitch, Vs + 2 * tx, lo, hi);
-    } else {
-      combine<DP, TI>(acc, Ps + r0 * kAtPitch, Vs + 2 * tx);
-    }
+    if (odd) combine_visible<DP, TI>(acc, Ps + r0 * kAtPitch, Vs + 2 * tx, -kAtCols, row_base + r0 + 1 - t0);
+    else combine<DP, TI>(acc, Ps + r0 * kAtPitch, Vs + 2 * tx);
   }
   T* ob = (T*)P.o + (int64_t)b * P.so.b + (int64_t)h * P.so.h;
 #pragma unroll
@@ -317,9 +316,11 @@ attn_bwd_dq_simt(const SimtParams P) {
   const int kv_end = P.causal ? min(row_base + ROWS, S) : S;
   for (int t0 = 0; t0 < kv_end; t0 += kAtCols) {
     __syncthreads();
-    const bool diagonal = P.causal && t0 + kAtCols > row_base + 1;
+    load_rows<T, DP, kAtCols>(Ks, kb, P.sk.s, t0, S, D, 1.f, P.vec);
     load_rows<T, DP, kAtCols>(Vs, vb, P.sv.s, t0, S, D, 1.f, P.vec);
-    const int odd = __syncthreads_or(load_rows<T, DP, kAtCols>(Ks, kb, P.sk.s, t0, S, D, 1.f, P.vec, diagonal));
+    __syncthreads();
+    bool odd = false;
+    if (P.causal && t0 + kAtCols > row_base + 1) odd = __syncthreads_or(tile_odd<DP>(Ks) | tile_odd<DP>(Vs));
     if (P.causal && t0 > warp_last) continue;
     float p[TI][4], dp[TI][4];
     dots<DP, TI>(p, Qs + r0 * (DP + 4), Ks + tx * (DP + 4));
@@ -337,19 +338,10 @@ attn_bwd_dq_simt(const SimtParams P) {
 #pragma unroll
     for (int i = 0; i < TI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool seen = !P.causal || t0 + tx + 16 * j <= row_base + r0 + 2 * i;        // (0 * NaN)
-        Ps[(r0 + 2 * i) * kAtPitch + tx + 16 * j] = seen ? p[i][j] * (dp[i][j] - drow[i]) * P.scale : 0.f;
-      }
+      for (int j = 0; j < 4; ++j) Ps[(r0 + 2 * i) * kAtPitch + tx + 16 * j] = p[i][j] * (dp[i][j] - drow[i]) * P.scale;
     __syncwarp();
-    if (diagonal && odd) {
-      int lo[TI], hi[TI];
-#pragma unroll
-      for (int i = 0; i < TI; ++i) { lo[i] = 0; hi[i] = row_base + r0 + 2 * i + 1 - t0; }
-      combine_visible<DP, TI>(acc, Ps + r0 * kAtPitch, Ks + 2 * tx, lo, hi);
-    } else {
-      combine<DP, TI>(acc, Ps + r0 * kAtPitch, Ks + 2 * tx);
-    }
+    if (odd) combine_visible<DP, TI>(acc, Ps + r0 * kAtPitch, Ks + 2 * tx, -kAtCols, row_base + r0 + 1 - t0);
+    else combine<DP, TI>(acc, Ps + r0 * kAtPitch, Ks + 2 * tx);
   }
   T* dqb = (T*)P.dq + (int64_t)b * P.sdq.b + (int64_t)h * P.sdq.h;
 #pragma unroll
@@ -392,18 +384,17 @@ attn_bwd_dkv_simt(const SimtParams P) {
     const T* gb = (const T*)P.d_o + (int64_t)b * P.sdo.b + (int64_t)hq * P.sdo.h;
     for (int t0 = q_begin; t0 < S; t0 += kAtCols) {
       __syncthreads();
-      const bool diagonal = P.causal && t0 < row_base + ROWS - 1;
-      bool odd = load_rows<T, DP, kAtCols>(Qs, qb, P.sq.s, t0, S, D, 1.f, P.vec, diagonal);
-      odd |= load_rows<T, DP, kAtCols>(Gs, gb, P.sdo.s, t0, S, D, 1.f, P.vec, diagonal);
+      load_rows<T, DP, kAtCols>(Qs, qb, P.sq.s, t0, S, D, 1.f, P.vec);
+      load_rows<T, DP, kAtCols>(Gs, gb, P.sdo.s, t0, S, D, 1.f, P.vec);
       if (threadIdx.x < kAtCols) {
         const int gi = t0 + threadIdx.x;
         Ls[threadIdx.x] = gi < S ? P.lse[bhq * S + gi] : 0.f;
         Ds[threadIdx.x] = gi < S ? P.delta[bhq * S + gi] : 0.f;
       }
-      odd = __syncthreads_or(odd) && diagonal;
-      int lo[TI], hi[TI];
-#pragma unroll
-      for (int i = 0; i < TI; ++i) { lo[i] = row_base + r0 + 2 * i - t0; hi[i] = kAtCols; }
+      __syncthreads();
+      bool odd = false;
+      if (P.causal && t0 < row_base + ROWS - 1)
+        odd = __syncthreads_or(tile_odd<DP>(Qs) | tile_odd<DP>(Gs) | !isfinite(Ds[threadIdx.x % kAtCols]));
       float p[TI][4], ds[TI][4];
       dots<DP, TI>(p, Ks + r0 * (DP + 4), Qs + tx * (DP + 4));
 #pragma unroll
@@ -417,7 +408,7 @@ attn_bwd_dkv_simt(const SimtParams P) {
         }
       }
       __syncwarp();
-      if (odd) combine_visible<DP, TI>(accv, Ps + r0 * kAtPitch, Gs + 2 * tx, lo, hi);
+      if (odd) combine_visible<DP, TI>(accv, Ps + r0 * kAtPitch, Gs + 2 * tx, row_base + r0 - t0, 3 * kAtCols);
       else combine<DP, TI>(accv, Ps + r0 * kAtPitch, Gs + 2 * tx);
       dots<DP, TI>(ds, Vs + r0 * (DP + 4), Gs + tx * (DP + 4));
       __syncwarp();
@@ -426,11 +417,10 @@ attn_bwd_dkv_simt(const SimtParams P) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int c = tx + 16 * j;
-          const bool seen = !P.causal || t0 + c >= row_base + r0 + 2 * i;
-          Ps[(r0 + 2 * i) * kAtPitch + c] = seen ? p[i][j] * (ds[i][j] - Ds[c]) * P.scale : 0.f;
+          Ps[(r0 + 2 * i) * kAtPitch + c] = p[i][j] * (ds[i][j] - Ds[c]) * P.scale;
         }
       __syncwarp();
-      if (odd) combine_visible<DP, TI>(acck, Ps + r0 * kAtPitch, Qs + 2 * tx, lo, hi);
+      if (odd) combine_visible<DP, TI>(acck, Ps + r0 * kAtPitch, Qs + 2 * tx, row_base + r0 - t0, 3 * kAtCols);
       else combine<DP, TI>(acck, Ps + r0 * kAtPitch, Qs + 2 * tx);
     }
   }
