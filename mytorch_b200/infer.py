@@ -2,7 +2,7 @@
 gpt2_trainer/gpt2.py:352-374 and nanochat_trainer/core/nanochat_gpt.py:301-340.
 
 A `Plan` describes a model's weights to the library: addresses and sizes. It is kept on the model and
-looked over by every forward: no module has had an attribute assigned since, the config, the blocks and
+looked over by every forward: no module has had an attribute assigned since, the sizes in the config, the blocks and
 the classes' forwards are the same, and every weight still holds the same array. Otherwise the model is
 walked and described anew, so replaced modules, weights, tables and options take effect at once. The
 plan holds weak references only, so it keeps no array of the model alive. Models that the call does not
@@ -32,6 +32,12 @@ def plain(module, cls):
 def methods(*classes):
     """The forwards (and Module.__call__) that the library call stands for, as they are at import."""
     return [(c, "forward", c.forward) for c in classes] + [(Module, "__call__", Module.__call__)]
+
+
+def config_of(model):
+    """What the descriptions read of a config, whatever kind of object that is."""
+    c = model.config
+    return [getattr(c, n, None) for n in ("embed_dim", "mlp_ratio", "vocab_size", "num_heads", "num_q_heads", "num_kv_heads")]
 
 
 def unpatched(known):
@@ -71,7 +77,7 @@ class Plan:
     then per block 16 in the order of `block_ptrs` in mytorch_b200.h; None where there is none."""
 
     def __init__(self, model, edits, sizes, tensors, known):
-        self.edits, self.config, self.known, self.ok = edits, dict(vars(model.config)), known, False
+        self.edits, self.config, self.known, self.ok = edits, config_of(model), known, False
         self.block_refs = [weakref.ref(b) for b in model.blocks]
         self.refs = [(weakref.ref(t), weakref.ref(t.data)) for t in tensors if isinstance(t, Tensor)]
         held = [t.data if isinstance(t, Tensor) else t for t in tensors]
@@ -104,7 +110,7 @@ class Plan:
         self.ok = True
 
     def current(self, model):
-        if self.edits != Module.edits or vars(model.config) != self.config or len(model.blocks) != len(self.block_refs) \
+        if self.edits != Module.edits or config_of(model) != self.config or len(model.blocks) != len(self.block_refs) \
                 or not unpatched(self.known):
             return False
         for b, r in zip(model.blocks, self.block_refs):

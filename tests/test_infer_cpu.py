@@ -148,6 +148,22 @@ def test_patched_classes_run_op_by_op(calls, monkeypatch):
     assert not forward(model)
 
 
+def test_configs_of_any_kind(calls):
+    """Attributes in slots or on the class are read like a dataclass's."""
+    plain = gpt2.GPT2Config(vocab_size=96, max_seq_len=32, embed_dim=128, num_blocks=2, num_heads=2)
+    names = list(vars(plain))
+    slots = type("Slots", (), {"__slots__": names})()
+    for n in names:
+        setattr(slots, n, getattr(plain, n))
+    held = type("Held", (), dict(vars(plain)))
+    for config, edit in ((slots, slots), (held(), held), (held, held)):
+        model = gpt2.GPT2(config)
+        assert forward(model) and forward(model)
+        edit.num_heads = 4
+        assert not forward(model)
+        edit.num_heads = 2
+
+
 def test_old_arrays_are_not_held(calls):
     model = gpt2_model()
     assert forward(model)
